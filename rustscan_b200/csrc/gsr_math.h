@@ -752,20 +752,6 @@ template <class F> GSR_HD F blend_alpha(F px, F py, F mx, F my, F ca, F cb, F cc
 // Colour accumulation C += max(c, 0) * w as one fused multiply-add.
 template <class F> GSR_HD F blend_accum(F C, F c, F w) { return gfma(gmax(c, F(0)), w, C); }
 
-// Padded half-widths of the box around the ellipse {0.5 d^T C d <= cut}
-// (C = conic): sqrt(2 cut (C^-1)_ii), determinant in double, widened by 0.1%
-// plus 0.01 px so that float rounding can never put a pixel of the true
-// ellipse outside it. Returns false (no box) for non-positive-definite
-// conics or non-finite input.
-GSR_HD bool footprint_box(float a, float b, float c, float cut, float& rx, float& ry) {
-  const double det = (double)a * (double)c - (double)b * (double)b;
-  if (!(det > 0.0) || !(a > 0.0f) || !(c > 0.0f) || !(cut > 0.0f)) return false;
-  const double q = 2.0 * (double)cut / det;
-  rx = (float)(sqrt(q * (double)c) * 1.001 + 0.01);
-  ry = (float)(sqrt(q * (double)a) * 1.001 + 0.01);
-  return rx == rx && ry == ry && rx < 3.0e38f && ry < 3.0e38f;
-}
-
 // A Gaussian whose sigma exceeds log(255 * opac) + kRejectMargin cannot pass
 // the alpha >= 1/255 test: its exact alpha is below (1/255) * exp(-1e-3),
 // far outside the few-ulp error of the float exp and log. Kernels use this

@@ -44,9 +44,7 @@ constexpr int kWalkBlocksPerSm = 24;
 // EMIT = false: count the passing tiles of every compact index (gid order).
 // EMIT = true: walk the Gaussians in depth order and write, for every
 // passing tile, the tile id as key and the compact index as value at the
-// Gaussian's scanned offset; then replace the record's tile box with the
-// footprint half-widths the rasterizer culls warp blocks with (negative: no
-// box, never cull).
+// Gaussian's scanned offset.
 // SLOTS (emission only): every box tile of a Gaussian has a slot at its
 // row-major position after the Gaussian's offset (offsets scanned from box
 // sizes, no counting walk); a passing tile writes its key there (packed, or
@@ -64,8 +62,7 @@ __global__ void __launch_bounds__(kWalkThreads, 5) tile_walk_kernel(ViewSet vs, 
   const TileShape ts{vs.tile_w, vs.tile_h};
   const uint32_t* perm = slice(b.perm, b.Vcap, v);
   const uint32_t* off = slice(b.offset, b.Vcap, v);
-  float4* rec_w = slice(b.rec, b.Vcap * 3, v);
-  const float4* rec = rec_w;
+  const float4* rec = slice(b.rec, b.Vcap * 3, v);
   uint32_t* count = slice(b.count, b.Vcap, v);
   uint32_t* keys = slice(b.isect_key_raw, b.Icap, v);
   uint32_t* vals = slice(b.isect_val_raw, b.Icap, v);
@@ -205,17 +202,7 @@ __global__ void __launch_bounds__(kWalkThreads, 5) tile_walk_kernel(ViewSet vs, 
       }
       __syncwarp();
     }
-    if (r < V) {
-      if (!EMIT) {
-        count[c] = S.run[lane];
-      } else {
-        float rx = -1.f, ry = -1.f;
-        if (!footprint_box(conic.x, conic.y, conic.z, thr + kRejectMargin, rx, ry)) rx = ry = -1.f;
-        float4* rw = rec_w + (size_t)c * 3 + 2;
-        rw->z = rx;
-        rw->w = ry;
-      }
-    }
+    if (!EMIT && r < V) count[c] = S.run[lane];
   }
   if (HIST) {
     __syncthreads();

@@ -5,12 +5,11 @@
 // warp owns an 8 x 4*PPL pixel block of the tile; each lane owns PPL pixels
 // of one column (rows y, y+4, ...), so the per-Gaussian terms a*dx*dx and
 // 2b*dx are formed once for all of them. The tile's depth-sorted list is staged in
-// shared memory batch by batch; while staging, every Gaussian's padded
-// axis-aligned box of its {sigma <= log(255*opacity) + 1e-3} ellipse
-// (footprint_box, written into the record by the emission kernel) gives a
-// bit per warp block it can reach.
+// shared memory batch by batch; while staging, the smallest sigma over each
+// warp block's rectangle gives a bit per block that the Gaussian's
+// {sigma <= log(255*opacity) + 1e-3} ellipse can reach (reached_blocks).
 // Each warp then walks, in order, only the Gaussians whose bit it holds
-// (ballot compaction into a per-warp list). The box is conservative and
+// (ballot compaction into a per-warp list). The test is conservative and
 // sigma is evaluated with the same expression tree as the oracle, so every
 // contributor decision is unchanged: culled Gaussians could not pass the
 // alpha >= 1/255 test (see kRejectMargin).
@@ -101,7 +100,7 @@ struct CostListView {
   uint32_t first[kCostLists];
 };
 __device__ __forceinline__ void load_cost_lists(const RasterArgs& a, CostListView* s) {
-  if (a.persist != 2) return;
+  if (!a.persist) return;
   if (threadIdx.x == 0) {
     uint32_t run = 0;
     for (int k = kCostLists - 1; k >= 0; --k) {
@@ -115,32 +114,31 @@ __device__ __forceinline__ void load_cost_lists(const RasterArgs& a, CostListVie
 
 // The next work item of this CTA (block-uniform; kNoItem when done). In
 // the grid schedule a CTA runs item blockIdx.x once; in the persistent one
-// thread 0 takes a ticket and reads the item at that place of the cost
-// order. The leading barrier keeps the previous item's shared state intact
-// until every thread is done with it (and publishes load_cost_lists).
-__device__ __forceinline__ uint32_t next_item(const RasterArgs& a, uint32_t round, uint32_t* s_item,
-                                              const CostListView* lists) {
+// thread 0 takes a ticket and reads the item at that place of the order: the
+// forward's sched_order, or the backward's cost lists. The leading barrier
+// keeps the previous item's shared state intact until every thread is done
+// with it (and publishes load_cost_lists).
+template <class At>
+__device__ __forceinline__ uint32_t take_item(const RasterArgs& a, uint32_t round, uint32_t* s_item, At at) {
   if (!a.persist) return round == 0 ? blockIdx.x : kNoItem;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const uint32_t slot = atomicAdd(a.b.sched_ticket, 1u);
-    uint32_t item = kNoItem;
-    if (slot < a.vs.total_tiles) {
-      if (a.persist == 1) {
-        item = a.b.sched_order[slot];
-      } else {
-        for (int k = kCostLists - 1; k >= 0; --k) {
-          if (slot - lists->first[k] < lists->count[k]) {
-            item = a.b.sched_lists[(size_t)k * a.b.sched_items_cap + (slot - lists->first[k])];
-            break;
-          }
-        }
-      }
-    }
-    *s_item = item;
-  }
+  if (threadIdx.x == 0) *s_item = at(atomicAdd(a.b.sched_ticket, 1u));
   __syncthreads();
   return *s_item;
+}
+__device__ __forceinline__ uint32_t next_item(const RasterArgs& a, uint32_t round, uint32_t* s_item) {
+  return take_item(a, round, s_item, [&](uint32_t slot) {
+    return slot < a.vs.total_tiles ? a.b.sched_order[slot] : kNoItem;
+  });
+}
+__device__ __forceinline__ uint32_t next_item(const RasterArgs& a, uint32_t round, uint32_t* s_item,
+                                              const CostListView* lists) {
+  return take_item(a, round, s_item, [&](uint32_t slot) {
+    for (int k = kCostLists - 1; k >= 0; --k)
+      if (slot - lists->first[k] < lists->count[k])
+        return a.b.sched_lists[(size_t)k * a.b.sched_items_cap + (slot - lists->first[k])];
+    return kNoItem;
+  });
 }
 
 // One block: the work items of a persistent forward in decreasing order of
@@ -184,29 +182,33 @@ template <int TW, int PPL> struct WarpBlock {
   __device__ static int y0(int w) { return (w / kWarpsX) * kRows; }
 };
 
-// Stages one Gaussian for the forward: its blend terms (colours clamped at
-// zero) plus the bit mask of warp blocks its padded footprint box overlaps
-// (half-widths written by the emission kernel into r2.zw; negative means no
-// box, never cull).
-template <int TW, int PPL, int NW>
-__device__ __forceinline__ uint32_t stage_one(const float4* rec, uint32_t c, float tx0, float ty0, float4& A, float4& B,
-                                              float4& Cc) {
-  const float4 r0 = rec[(size_t)c * 3 + 0];
-  const float4 r1 = rec[(size_t)c * 3 + 1];
-  const float4 r2 = rec[(size_t)c * 3 + 2];
-  A = make_float4(r0.x, r0.y, r0.z, 2.f * r0.w);  // 2b is exact
-  B = make_float4(r1.x, r2.y + kRejectMargin, r1.y, 0.f);
-  Cc = make_float4(fmaxf(r1.z, 0.f), fmaxf(r1.w, 0.f), fmaxf(r2.x, 0.f), 0.f);
-  const float rx = r2.z, ry = r2.w;
-  if (!(rx >= 0.f) || !(ry >= 0.f)) return (1u << NW) - 1u;
-  uint32_t mask = 0;
-  constexpr float kSpanY = (float)(4 * PPL - 1);
+// The 8x8 warp blocks of a tile at (tx0, ty0) that a Gaussian can reach: bit
+// w set unless sigma exceeds the cut over the whole rectangle of block w's
+// pixel centres. The smallest value of a positive-definite quadratic over a
+// rectangle that does not hold its centre lies on an edge facing the centre,
+// so two clamped edge minima give it. The test errs on the side of keeping:
+// sigma as the pixels evaluate it (and this minimum) is within 10 units of
+// 2^-24 of (a dx^2 + c dy^2), which the last term covers threefold, and the
+// cut itself lies kRejectMargin above any sigma that can contribute. A conic
+// that float arithmetic cannot tell from an indefinite one, or a value that is
+// not a number, keeps every block.
+template <int TW, int NW>
+__device__ __forceinline__ uint32_t reached_blocks(float x, float y, float a, float b, float c, float cut, float tx0,
+                                                   float ty0) {
+  uint32_t mask = (1u << NW) - 1u;
+  if (!(a > 0.f && c > 0.f && a * c > b * b * (1.f + 5e-7f))) return mask;
+  const float ka = __fdividef(-b, a), kc = __fdividef(-b, c), b2 = 2.f * b;
 #pragma unroll
   for (int w = 0; w < NW; ++w) {
-    const float bx0 = tx0 + (float)WarpBlock<TW, PPL>::x0(w) + 0.5f;
-    const float by0 = ty0 + (float)WarpBlock<TW, PPL>::y0(w) + 0.5f;
-    const bool out = (r0.x + rx < bx0) || (r0.x - rx > bx0 + 7.f) || (r0.y + ry < by0) || (r0.y - ry > by0 + kSpanY);
-    if (!out) mask |= 1u << w;
+    // Offsets mean - centre over the block's columns and rows.
+    const float x1 = x - (tx0 + (float)(8 * (w % (TW / 8))) + 0.5f), x0 = x1 - 7.f;
+    const float y1 = y - (ty0 + (float)(8 * (w / (TW / 8))) + 0.5f), y0 = y1 - 7.f;
+    const float nx = fminf(fmaxf(0.f, x0), x1), ny = fminf(fmaxf(0.f, y0), y1);
+    const float ey = fminf(fmaxf(kc * nx, y0), y1), ex = fminf(fmaxf(ka * ny, x0), x1);
+    const float q1 = fmaf(fmaf(a, nx, b2 * ey), nx, c * ey * ey);
+    const float q2 = fmaf(fmaf(c, ny, b2 * ex), ny, a * ex * ex);
+    const float fx = fmaxf(fabsf(x0), fabsf(x1)), fy = fmaxf(fabsf(y0), fabsf(y1));
+    if (0.5f * fminf(q1, q2) - 2e-6f * (a * fx * fx + c * fy * fy) > cut) mask &= ~(1u << w);
   }
   return mask;
 }
@@ -282,45 +284,67 @@ __device__ __forceinline__ float2 blend_exp2(float2 sigma) {
   return make_float2(__uint_as_float(__float_as_uint(p.x) + ex), __uint_as_float(__float_as_uint(p.y) + ey));
 }
 
-// Per-entry terms of a forward step for one pixel pair.
-struct FwdPre {
-  float2 sg;       // sigma of both pixels
-  float opac;
-  float ax, ay;    // alpha of both pixels
-  bool l0, l1;     // within the cut
-  bool c0, c1;     // contributes (before the pixel-state gate)
+// A list entry as the forward stages it. Values that both pixels of a pair
+// take lie twice side by side, so that a load brings them as the register
+// pair a two-wide operation wants.
+struct __align__(16) FwdEntry {
+  float x, a, b2, cut;    // mean x, conic a, 2 conic b (exact), reject cut
+  float2 y, c;            // mean y, conic c
+  float2 opac, r;         // opacity, max(red, 0)
+  float2 g, b;            // max(green, 0), max(blue, 0)
+  uint32_t last;          // list index + 1
+  uint8_t hit[4];         // warp block w took the entry
+  uint32_t cidx, pad;
 };
+// Entries a warp evaluates together. Two cost nothing on large launches but
+// 2% on a launch of 300 tiles, where few warps hide each other's latency.
+constexpr int kFwdUnroll = 4;
+// Resident threads per SM the register bound allows (768: 80 registers): 8
+// views of 1280x720 blend in 0.832 ms, in 0.844 at 640 and 0.830 with more
+// spills at 896.
+constexpr int kFwdThreadsPerSm = 768;
 
-template <int TW, int TH, int PPL, int BATCH>
-__global__ void __launch_bounds__(TW* TH / PPL) raster_fwd_kernel(RasterArgs a) {
-  static_assert(PPL % 2 == 0, "pixels per lane come in pairs");
-  static_assert(TH % (4 * PPL) == 0 && (TW * TH / PPL) % 32 == 0, "warp blocks tile the tile");
-  constexpr int NT = TW * TH / PPL;
+// One CTA per tile, a warp per 8x8 block, a lane per pixel pair (rows y and
+// y + 4 of one column). Per batch every entry is staged once with the blocks
+// it can reach; each warp walks the entries of its block in list order, four
+// at a time. The four sigmas, exponentials and contribution tests are
+// independent of the pixel state and run as one straight-line block, so their
+// latencies overlap; the four blends then follow in order. No branch depends
+// on a pixel: a pixel that does not take an entry blends with alpha 0, which
+// leaves its colour and transmittance bit for bit unchanged, and a saturated
+// pixel (transmittance below 1e-4) takes nothing. What bounds it is
+// instruction issue (0.71 of the slots) and, on launches of few tiles, the
+// latency of the longest tile. Against a walk of two entries with a vote and
+// a branch each, over blocks culled by the footprint's bounding box: 8 views
+// of 1280x720 over 1M Gaussians 1.10 -> 0.83 ms (135M -> 90M warp instructions
+// a view), one view of 320x240 over 74k 0.193 -> 0.104 ms.
+template <int TW, int TH, int BATCH>
+__global__ void __launch_bounds__(TW* TH / 2, kFwdThreadsPerSm / (TW * TH / 2)) raster_fwd_kernel(RasterArgs a) {
+  constexpr int NT = TW * TH / 2;
   constexpr int NW = NT / 32;
-  constexpr int NP = PPL / 2;
-  __shared__ float4 s_a[BATCH];  // x, y, conic a, 2 conic b
-  __shared__ float4 s_b[BATCH];  // conic c, reject cut, opacity, -
-  __shared__ float4 s_c[BATCH];  // max(r,0), max(g,0), max(b,0), -
-  __shared__ uint32_t s_cidx[BATCH];
+  static_assert(NW <= 4 && TW % 8 == 0 && TH % 8 == 0, "hit bits of at most four 8x8 blocks");
+  __shared__ FwdEntry s_e[BATCH + 1];  // the last one is never taken: it pads the lists
   __shared__ uint8_t s_mask[BATCH];
-  __shared__ uint8_t s_hit[NW][BATCH];  // warp w took entry j
-  __shared__ uint16_t s_list[NW][BATCH];
+  __shared__ __align__(8) uint16_t s_list[NW][BATCH + kFwdUnroll];  // byte offsets into s_e
   __shared__ uint32_t s_item;
   __shared__ uint32_t s_work;
-  __shared__ CostListView s_lists;
-  if (threadIdx.x == 0) s_work = 0u;
-  load_cost_lists(a, &s_lists);
+  if (threadIdx.x == 0) {
+    s_work = 0u;
+    s_e[BATCH] = FwdEntry{};  // sigma 0, opacity 0: alpha 0
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint16_t* list = s_list[warp];
   for (uint32_t round = 0;; ++round) {
-    const uint32_t item = next_item(a, round, &s_item, &s_lists);
+    const uint32_t item = next_item(a, round, &s_item);
     if (item == kNoItem) break;
     const uint32_t v = find_view(a.vs, item);
     const ViewDesc& vd = a.vs.views[v];
     const uint32_t t = item - vd.tile_base;
     const uint32_t tx = t % vd.tiles_x, ty = t / vd.tiles_x;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t px = tx * TW + WarpBlock<TW, PPL>::x0(warp) + (lane & 7);
-    const uint32_t pyb = ty * TH + WarpBlock<TW, PPL>::y0(warp) + (lane >> 3);
+    const uint32_t px = tx * TW + WarpBlock<TW, 2>::x0(warp) + (lane & 7);
+    const uint32_t py = ty * TH + WarpBlock<TW, 2>::y0(warp) + (lane >> 3);
     const float pcx = (float)px + 0.5f;
+    const float2 npcy = make_float2(-((float)py + 0.5f), -((float)(py + 4) + 0.5f));
     const uint32_t* ranges = slice(a.b.ranges, 2 * a.b.Tcap, v);
     const uint32_t s0 = ranges[2 * t], s1 = ranges[2 * t + 1];
     const uint32_t* vals = isect_index_src(a.b, v);
@@ -329,161 +353,130 @@ __global__ void __launch_bounds__(TW* TH / PPL) raster_fwd_kernel(RasterArgs a) 
     uint8_t* vis = slice(a.b.visible_c, a.b.Vcap, v);
     uint8_t* hitw = slice(a.b.hitw, a.b.Icap, v);
     const float tx0 = (float)(tx * TW), ty0 = (float)(ty * TH);
-    // Pixel q = 2k + h sits at row pyb + 4q and is half h of pair k.
-    float2 T[NP], C0[NP], C1[NP], C2[NP], npcy[NP];
-    uint32_t last[PPL], nc[PPL];  // a pixel that saturates stops at its last contributor
-    bool done[PPL];
-    bool all_done = true;
-  #pragma unroll
-    for (int k = 0; k < NP; ++k) {
-      T[k] = f2(1.f);
-      C0[k] = C1[k] = C2[k] = f2(0.f);
-      npcy[k] = make_float2(-((float)(pyb + 8 * k) + 0.5f), -((float)(pyb + 8 * k + 4) + 0.5f));
-    }
-  #pragma unroll
-    for (int q = 0; q < PPL; ++q) {
-      const uint32_t py = pyb + 4 * q;
-      last[q] = nc[q] = 0;
-      done[q] = !(px < vd.w && py < vd.h);
-      all_done = all_done && done[q];
-    }
+    const bool in0 = px < vd.w && py < vd.h, in1 = px < vd.w && py + 4 < vd.h;
+    // A pixel outside the image starts saturated.
+    float2 T = make_float2(in0 ? 1.f : 0.f, in1 ? 1.f : 0.f);
+    float2 C0 = f2(0.f), C1 = f2(0.f), C2 = f2(0.f);
+    uint32_t last0 = 0, last1 = 0, nc0 = 0, nc1 = 0;
+    struct Raw {
+      uint32_t c;
+      float4 r0, r1, r2;
+    };
+    auto load = [&](uint32_t i) {
+      Raw r;
+      r.c = vals[i] & vmask;
+      r.r0 = rec[(size_t)r.c * 3 + 0];
+      r.r1 = rec[(size_t)r.c * 3 + 1];
+      r.r2 = rec[(size_t)r.c * 3 + 2];
+      return r;
+    };
+    auto stage = [&](uint32_t j, uint32_t i, const Raw& r) {
+      const float cut = r.r2.y + kRejectMargin;
+      FwdEntry& E = s_e[j];
+      E.x = r.r0.x;
+      E.a = r.r0.z;
+      E.b2 = 2.f * r.r0.w;
+      E.cut = cut;
+      E.y = f2(r.r0.y);
+      E.c = f2(r.r1.x);
+      E.opac = f2(r.r1.y);
+      E.r = f2(fmaxf(r.r1.z, 0.f));
+      E.g = f2(fmaxf(r.r1.w, 0.f));
+      E.b = f2(fmaxf(r.r2.x, 0.f));
+      E.last = i + 1;
+      *reinterpret_cast<uint32_t*>(E.hit) = 0u;
+      E.cidx = r.c;
+      s_mask[j] = (uint8_t)reached_blocks<TW, NW>(r.r0.x, r.r0.y, r.r0.z, r.r0.w, r.r1.x, cut, tx0, ty0);
+    };
     for (uint32_t b0 = s0; b0 < s1; b0 += BATCH) {
       const uint32_t nb = min((uint32_t)BATCH, s1 - b0);
+      for (uint32_t j = threadIdx.x; j < nb; j += NT) stage(j, b0 + j, load(b0 + j));
       __syncthreads();
-      for (uint32_t j = threadIdx.x; j < nb; j += NT) {
-        const uint32_t c = vals[b0 + j] & vmask;
-        float4 A, B, Cc;
-        s_mask[j] = (uint8_t)stage_one<TW, PPL, NW>(rec, c, tx0, ty0, A, B, Cc);
-        s_a[j] = A;
-        s_b[j] = B;
-        s_c[j] = Cc;
-        s_cidx[j] = c;
-  #pragma unroll
-        for (int w = 0; w < NW; ++w) s_hit[w][j] = 0;
-      }
-      __syncthreads();
-      if (!__all_sync(0xffffffffu, all_done)) {
-        const int cnt = build_list(s_mask, nb, 1u << warp, lane, s_list[warp]);
-        // Entries go two at a time: the sigma, cut test, exponential and
-        // contribution test of both (independent of the pixel state) form one
-        // straight-line block whose chains interleave; the blends then apply
-        // in list order, the second gated by the pixel state the first left.
-        for (int e = 0; e < cnt; e += 2) {
-          const bool two = e + 1 < cnt;  // warp-uniform
-          const uint32_t jj[2] = {s_list[warp][e], two ? s_list[warp][e + 1] : s_list[warp][e]};
-          FwdPre pre[2][NP];
-          uint32_t need = 0;
-  #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const float4 A = s_a[jj[u]];
-            const float4 B = s_b[jj[u]];
-            const float dx = esub(A.x, pcx);
-            const float t1 = emul(emul(A.z, dx), dx);
-            const float t2 = emul(A.w, dx);
-  #pragma unroll
-            for (int k = 0; k < NP; ++k) {
-              FwdPre& q = pre[u][k];
-              const float2 dy = add2(f2(A.y), npcy[k]);
-              q.sg = sigma2(t1, t2, dy, B.x);
-              q.l0 = !(q.sg.x > B.y);
-              q.l1 = !(q.sg.y > B.y);
-              q.opac = B.z;
-              if (__any_sync(0xffffffffu, (q.l0 && !done[2 * k]) || (q.l1 && !done[2 * k + 1])) && (u == 0 || two))
-                need |= 1u << (u * NP + k);
-            }
+      if (!__all_sync(0xffffffffu, T.x < 1e-4f && T.y < 1e-4f)) {
+        // The entries of this warp's block in list order, padded to a multiple
+        // of the unroll.
+        uint32_t cnt = 0;
+        for (uint32_t base = 0; base < nb; base += 32) {
+          const uint32_t j = base + lane;
+          const bool bit = j < nb && ((s_mask[j] >> warp) & 1u);
+          const uint32_t bal = __ballot_sync(0xffffffffu, bit);
+          if (bit) list[cnt + __popc(bal & ((1u << lane) - 1u))] = (uint16_t)(j * sizeof(FwdEntry));
+          cnt += __popc(bal);
+        }
+        if (lane < kFwdUnroll) list[cnt + lane] = (uint16_t)(BATCH * sizeof(FwdEntry));
+        __syncwarp();
+        for (uint32_t e = 0; e < cnt; e += kFwdUnroll) {
+          const uint2 off2 = *reinterpret_cast<const uint2*>(list + e);
+          const uint32_t off[kFwdUnroll] = {off2.x & 0xffffu, off2.x >> 16, off2.y & 0xffffu, off2.y >> 16};
+          float2 al[kFwdUnroll];
+          bool k0[kFwdUnroll], k1[kFwdUnroll];
+#pragma unroll
+          for (int u = 0; u < kFwdUnroll; ++u) {
+            const FwdEntry& E = *reinterpret_cast<const FwdEntry*>(reinterpret_cast<const char*>(s_e) + off[u]);
+            const float dx = esub(E.x, pcx);
+            const float t1 = emul(emul(E.a, dx), dx);
+            const float t2 = emul(E.b2, dx);
+            const float2 dy = add2(E.y, npcy);
+            const float2 in = make_float2(fmaf(t2, dy.x, t1), fmaf(t2, dy.y, t1));
+            const float2 sg = mul2(f2(0.5f), fma2(mul2(E.c, dy), dy, in));  // sigma, as blend_sigma_shared
+            const float2 og = mul2(E.opac, blend_exp2(sg));
+            al[u] = make_float2(fminf(0.999f, og.x), fminf(0.999f, og.y));
+            // 0 <= sigma <= cut in one unsigned comparison of the bits (sigma is
+            // never -0; a negative one has the sign bit set) and alpha >= 1/255,
+            // as blend_alpha_of decides.
+            const uint32_t cut = __float_as_uint(E.cut);
+            k0[u] = __float_as_uint(sg.x) <= cut && al[u].x >= (float)(1.0 / 255.0);
+            k1[u] = __float_as_uint(sg.y) <= cut && al[u].y >= (float)(1.0 / 255.0);
           }
-          // blend_alpha_of (sigma >= 0 and alpha >= 1/255) and the blend of
-          // entry u, pair k. A pixel that does not take the Gaussian blends
-          // with alpha 0, which leaves its colour and transmittance bit for bit
-          // unchanged.
-          auto alpha = [&](FwdPre& q) {
-            const float2 og = mul2(f2(q.opac), blend_exp2(q.sg));
-            q.ax = fminf(0.999f, og.x);
-            q.ay = fminf(0.999f, og.y);
-            q.c0 = q.l0 && q.sg.x >= 0.f && q.ax >= (float)(1.0 / 255.0);
-            q.c1 = q.l1 && q.sg.y >= 0.f && q.ay >= (float)(1.0 / 255.0);
-          };
-          auto blend = [&](int u, int k) {
-            const FwdPre& q = pre[u][k];
-            const bool c0 = q.c0 && !done[2 * k], c1 = q.c1 && !done[2 * k + 1];
-            if (!(c0 || c1)) return;
-            const uint32_t j = jj[u];
-            const float2 am = make_float2(c0 ? q.ax : 0.f, c1 ? q.ay : 0.f);
-            const float4 Cc = s_c[j];
-            const float2 w = mul2(am, T[k]);
-            C0[k] = fma2(f2(Cc.x), w, C0[k]);  // blend_accum; Cc was clamped at staging
-            C1[k] = fma2(f2(Cc.y), w, C1[k]);
-            C2[k] = fma2(f2(Cc.z), w, C2[k]);
-            T[k] = mul2(T[k], add2(f2(1.f), neg2(am)));
-            s_hit[warp][j] = 1;
+#pragma unroll
+          for (int u = 0; u < kFwdUnroll; ++u) {
+            FwdEntry& E = *reinterpret_cast<FwdEntry*>(reinterpret_cast<char*>(s_e) + off[u]);
+            const bool c0 = k0[u] && !(T.x < 1e-4f), c1 = k1[u] && !(T.y < 1e-4f);
+            const float2 am = make_float2(c0 ? al[u].x : 0.f, c1 ? al[u].y : 0.f);
+            const float2 w = mul2(am, T);
+            C0 = fma2(E.r, w, C0);  // blend_accum; the colours were clamped at staging
+            C1 = fma2(E.g, w, C1);
+            C2 = fma2(E.b, w, C2);
+            T = mul2(T, add2(f2(1.f), neg2(am)));
+            if (c0 || c1) E.hit[warp] = 1;
             if (c0) {
-              last[2 * k] = b0 + j + 1;
-              ++nc[2 * k];
-              if (T[k].x < 1e-4f) done[2 * k] = true;
+              last0 = E.last;
+              ++nc0;
             }
             if (c1) {
-              last[2 * k + 1] = b0 + j + 1;
-              ++nc[2 * k + 1];
-              if (T[k].y < 1e-4f) done[2 * k + 1] = true;
+              last1 = E.last;
+              ++nc1;
             }
-          };
-          static_assert(NP == 1, "the forward runs one pixel pair per lane");
-          if (need == 3u) {
-            alpha(pre[0][0]);
-            alpha(pre[1][0]);
-            blend(0, 0);
-            blend(1, 0);
-          } else if (need == 1u) {
-            alpha(pre[0][0]);
-            blend(0, 0);
-          } else if (need == 2u) {
-            alpha(pre[1][0]);
-            blend(1, 0);
           }
-          all_done = true;
-  #pragma unroll
-          for (int q = 0; q < PPL; ++q) all_done = all_done && done[q];
-          if (__all_sync(0xffffffffu, all_done)) break;
+          if (__all_sync(0xffffffffu, T.x < 1e-4f && T.y < 1e-4f)) break;
         }
       }
       __syncthreads();
       for (uint32_t j = threadIdx.x; j < nb; j += NT) {
-        uint32_t bits = 0;
-  #pragma unroll
-        for (int w = 0; w < NW; ++w) bits |= (uint32_t)s_hit[w][j] << w;
-        hitw[b0 + j] = (uint8_t)bits;  // bit w: the 8x8 block of warp w
-        if (bits) vis[s_cidx[j]] = 1;
+        const uint32_t h = *reinterpret_cast<const uint32_t*>(s_e[j].hit);
+        hitw[b0 + j] = (uint8_t)((h | (h >> 7) | (h >> 14) | (h >> 21)) & 0xfu);  // bit w: the 8x8 block of warp w
+        if (h) vis[s_e[j].cidx] = 1;
       }
-      if (__syncthreads_and(all_done)) break;
+      if (__syncthreads_and(T.x < 1e-4f && T.y < 1e-4f)) break;
     }
     float4* out = reinterpret_cast<float4*>(a.out_rgba) + vd.pix_base;
-  #pragma unroll
-    for (int q = 0; q < PPL; ++q) {
-      const uint32_t py = pyb + 4 * q;
-      if (!(px < vd.w && py < vd.h)) continue;
-      const size_t pix = (size_t)py * vd.w + px;
-      const int k = q / 2;
-      const float Tq = (q & 1) ? T[k].y : T[k].x;
-      const float c0 = (q & 1) ? C0[k].y : C0[k].x;
-      const float c1 = (q & 1) ? C1[k].y : C1[k].x;
-      const float c2 = (q & 1) ? C2[k].y : C2[k].x;
+    auto finish = [&](uint32_t row, float Tq, float c0, float c1, float c2, uint32_t last, uint32_t nc) {
+      const size_t pix = (size_t)row * vd.w + px;
       out[pix] = make_float4(c0 + Tq * a.bg[0], c1 + Tq * a.bg[1], c2 + Tq * a.bg[2], 1.f - Tq);
       slice(a.b.tfinal, a.b.Pcap, v)[pix] = Tq;
-      slice(a.b.last, a.b.Pcap, v)[pix] = last[q];
-      slice(a.b.ncontrib, a.b.Pcap, v)[pix] = nc[q];
-      slice(a.b.nvisit, a.b.Pcap, v)[pix] = (done[q] ? last[q] : s1) - s0;
-    }
+      slice(a.b.last, a.b.Pcap, v)[pix] = last;
+      slice(a.b.ncontrib, a.b.Pcap, v)[pix] = nc;
+      slice(a.b.nvisit, a.b.Pcap, v)[pix] = (Tq < 1e-4f ? last : s1) - s0;  // a saturated pixel stopped there
+    };
+    if (in0) finish(py, T.x, C0.x, C1.x, C2.x, last0, nc0);
+    if (in1) finish(py + 4, T.y, C0.y, C1.y, C2.y, last1, nc1);
     // The backward's cost of this item: list entries up to the tile's
     // largest last contributor.
-    uint32_t ml = 0;
-#pragma unroll
-    for (int q = 0; q < PPL; ++q) ml = max(ml, last[q]);
-    ml = __reduce_max_sync(0xffffffffu, ml);
+    const uint32_t ml = __reduce_max_sync(0xffffffffu, max(last0, last1));
     if (lane == 0 && ml) atomicMax(&s_work, ml);
     __syncthreads();
     if (threadIdx.x == 0) {
-      const uint32_t cost = s_work > s0 ? s_work - s0 : 0u;
-      const uint32_t k = cost_bucket(cost);
+      const uint32_t k = cost_bucket(s_work > s0 ? s_work - s0 : 0u);
       a.b.sched_lists[(size_t)k * a.b.sched_items_cap + atomicAdd(a.b.sched_lcount + k, 1u)] = item;
       s_work = 0u;
     }
@@ -602,7 +595,7 @@ struct BwdAcc {
 
 // The first part of a reverse-walk step for both pixels of a pair: the
 // offsets and sigma, and whether each pixel can take the Gaussian at all
-// (it is before its last contributor and sigma is within the cut).
+// (it is before its last contributor and sigma is in [0, cut]).
 struct PairPre {
   float2 dy, sg;
   bool l0, l1;
@@ -613,8 +606,10 @@ __device__ __forceinline__ PairPre bwd_pair_pre(const BwdPair& p, float2 npcy, u
   const bool in0 = s < p.last0, in1 = s < p.last1;
   q.dy = add2(f2(A.y), npcy);
   q.sg = sigma2(t1, t2, q.dy, B.x);
-  q.l0 = in0 && !(q.sg.x > B.y);
-  q.l1 = in1 && !(q.sg.y > B.y);
+  // 0 <= sigma <= cut in one unsigned comparison, as in the forward.
+  const uint32_t cut = __float_as_uint(B.y);
+  q.l0 = in0 && __float_as_uint(q.sg.x) <= cut;
+  q.l1 = in1 && __float_as_uint(q.sg.y) <= cut;
   return q;
 }
 
@@ -634,8 +629,8 @@ __device__ __forceinline__ void bwd_pair_rest(BwdPair& p, const PairPre& q, floa
   const float2 gs = blend_exp2(q.sg);
   const float2 og = mul2(f2(B.z), gs);
   const float ax = fminf(0.999f, og.x), ay = fminf(0.999f, og.y);
-  const bool c0 = q.l0 && q.sg.x >= 0.f && ax >= (float)(1.0 / 255.0);
-  const bool c1 = q.l1 && q.sg.y >= 0.f && ay >= (float)(1.0 / 255.0);
+  const bool c0 = q.l0 && ax >= (float)(1.0 / 255.0);
+  const bool c1 = q.l1 && ay >= (float)(1.0 / 255.0);
   const bool sk0 = REF && p.T.x <= 1e-4f, sk1 = REF && p.T.y <= 1e-4f;
   const float2 al = make_float2(ax, ay);
   const float2 am = make_float2(c0 ? ax : 0.f, c1 ? ay : 0.f);
@@ -1231,13 +1226,13 @@ cudaError_t launch_items(int threads, const RasterArgs& a, int num_sms, cudaStre
   return cudaGetLastError();
 }
 
-template <int TW, int TH, int PPL>
+template <int TW, int TH>
 cudaError_t launch_fwd_shape(const RasterArgs& a, uint32_t batch, int num_sms, cudaStream_t st) {
-  constexpr int NT = TW * TH / PPL;
+  constexpr int NT = TW * TH / 2;
   switch (pick_batch(batch, 128)) {
-    case 64: return launch_items<raster_fwd_kernel<TW, TH, PPL, 64>>(NT, a, num_sms, st);
-    case 128: return launch_items<raster_fwd_kernel<TW, TH, PPL, 128>>(NT, a, num_sms, st);
-    default: return launch_items<raster_fwd_kernel<TW, TH, PPL, 256>>(NT, a, num_sms, st);
+    case 64: return launch_items<raster_fwd_kernel<TW, TH, 64>>(NT, a, num_sms, st);
+    case 128: return launch_items<raster_fwd_kernel<TW, TH, 128>>(NT, a, num_sms, st);
+    default: return launch_items<raster_fwd_kernel<TW, TH, 256>>(NT, a, num_sms, st);
   }
 }
 template <int TW, int TH, int PPL, bool REF>
@@ -1283,14 +1278,14 @@ void raster_warm_up(uint32_t tile_w, uint32_t tile_h, uint32_t batch, int num_sm
   for (int ref = 0; ref < 2; ++ref) {
     a.ref_mode = ref;
     if (tile_w == 16 && tile_h == 16) {
-      (void)launch_fwd_shape<16, 16, kFwdPPL>(a, batch, num_sms, nullptr);
+      (void)launch_fwd_shape<16, 16>(a, batch, num_sms, nullptr);
       (void)launch_bwd_16(a, batch, num_sms, nullptr);
       (void)launch_bwd_shape<16, 16, kBwdPPL16>(a, batch, num_sms, nullptr);
     } else if (tile_w == 8 && tile_h == 8) {
-      (void)launch_fwd_shape<8, 8, kFwdPPL>(a, batch, num_sms, nullptr);
+      (void)launch_fwd_shape<8, 8>(a, batch, num_sms, nullptr);
       (void)launch_bwd_shape<8, 8, kBwdPPL>(a, batch, num_sms, nullptr);
     } else if (tile_w == 32 && tile_h == 8) {
-      (void)launch_fwd_shape<32, 8, kFwdPPL>(a, batch, num_sms, nullptr);
+      (void)launch_fwd_shape<32, 8>(a, batch, num_sms, nullptr);
       (void)launch_bwd_shape<32, 8, kBwdPPL>(a, batch, num_sms, nullptr);
     }
   }
@@ -1317,9 +1312,9 @@ cudaError_t launch_raster_fwd(const ViewSet& vs, FwdBufs& b, const float* bg, fl
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  if (vs.tile_w == 16 && vs.tile_h == 16) return launch_fwd_shape<16, 16, kFwdPPL>(a, vs.batch, s.num_sms, st);
-  if (vs.tile_w == 8 && vs.tile_h == 8) return launch_fwd_shape<8, 8, kFwdPPL>(a, vs.batch, s.num_sms, st);
-  if (vs.tile_w == 32 && vs.tile_h == 8) return launch_fwd_shape<32, 8, kFwdPPL>(a, vs.batch, s.num_sms, st);
+  if (vs.tile_w == 16 && vs.tile_h == 16) return launch_fwd_shape<16, 16>(a, vs.batch, s.num_sms, st);
+  if (vs.tile_w == 8 && vs.tile_h == 8) return launch_fwd_shape<8, 8>(a, vs.batch, s.num_sms, st);
+  if (vs.tile_w == 32 && vs.tile_h == 8) return launch_fwd_shape<32, 8>(a, vs.batch, s.num_sms, st);
   return cudaErrorInvalidValue;
 }
 
