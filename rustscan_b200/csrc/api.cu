@@ -160,8 +160,13 @@ gsr_status allocate(gsr_ctx* c) {
             dalloc(c, &b.ncontrib, nv * P) && dalloc(c, &b.nvisit, nv * P) && dalloc(c, &b.visible_c, nv * V) &&
             dalloc(c, &b.sgrad, nv * V * 3) && dalloc(c, &b.pair, nv * V * 6) && dalloc(c, &b.vcount, nv * 4) &&
             dalloc(c, &b.tile_hist, nv * T) && dalloc(c, &b.hitw, nv * I) && dalloc(c, &b.sched_order, nv * T) &&
-            dalloc(c, &b.sched_lists, 33 * nv * T) && dalloc(c, &b.sched_lcount, 33) && dalloc(c, &b.sched_ticket, 1);
-  b.sched_items_cap = nv * T;
+            dalloc(c, &b.sched_lcount, 32) && dalloc(c, &b.sched_ticket, 1);
+  // Backward work items: the tiles, or the segments of a launch of few tiles.
+  b.sched_items_cap = std::max<uint64_t>(nv * T, kSegItems);
+  ok = ok && dalloc(c, &b.sched_lists, 32 * b.sched_items_cap);
+  b.seg_k = 1;
+  b.ckpt = nullptr;
+  if (cfg.tile_w == 16 && cfg.tile_h == 16) ok = ok && dalloc(c, &b.ckpt, (uint64_t)kSegItems * 256);
   b.proj_parts_cap = (uint32_t)((N + kProjBlock - 1) / kProjBlock);
   ok = ok && dalloc(c, &b.vis_bits, nv * b.proj_parts_cap * 8) && dalloc(c, &b.blk_count, nv * b.proj_parts_cap) &&
        dalloc(c, &b.blk_base, nv * b.proj_parts_cap);
@@ -195,7 +200,7 @@ gsr_status allocate(gsr_ctx* c) {
       cudaMemset(c->s.ctl, 0, sizeof(LookbackCtl)) != cudaSuccess ||
       cudaMemset(c->s.status, 0, sizeof(DevStatus)) != cudaSuccess ||
       cudaMemset(b.vcount, 0, sizeof(uint32_t) * 4 * nv) != cudaSuccess ||
-      cudaMemset(b.sched_lcount, 0, sizeof(uint32_t) * 33) != cudaSuccess)
+      cudaMemset(b.sched_lcount, 0, sizeof(uint32_t) * 32) != cudaSuccess)
     return cuda_fail(c, cudaGetLastError(), "cudaMemset");
   raster_warm_up(cfg.tile_w, cfg.tile_h, cfg.batch, c->num_sms);
   return GSR_OK;

@@ -45,10 +45,12 @@ struct FwdBufs {
   uint32_t* inv_perm;      // [I] emission index -> sorted position (deterministic mode)
   uint32_t* vcount;        // [4] visible, intersections (clamped), intersections required, pad
   uint32_t* sched_order;   // [views * Tcap] persistent forward: work items in issue order
-  uint32_t* sched_lists;   // [33][sched_items_cap] work items by the bit length of their backward cost
-  uint32_t* sched_lcount;  // [33] items in each of those lists (appended by the forward)
+  uint32_t* sched_lists;   // [32][sched_items_cap] work items by the bit length of their backward cost
+  uint32_t* sched_lcount;  // [32] items in each of those lists (appended by the forward)
   uint32_t* sched_ticket;  // [1] next ticket a persistent raster CTA takes
   uint64_t sched_items_cap;
+  float4* ckpt;            // [kSegItems][256] per (tile, segment) and pixel: transmittance after it, colour behind it
+  uint32_t seg_k;          // segments per tile of the last forward (1: no checkpoints)
   uint64_t Vcap, Ncap, Icap, Tcap, Pcap;
   uint32_t pack_bits;      // > 0: intersections are packed keys (see isect_key), else (tile, index) pairs
   bool slots;              // slot layout: one key per box tile, sentinel keys last; vcount[3] = keys sorted
@@ -72,6 +74,10 @@ struct ViewSet {
   uint32_t max_tiles;     // max over views
   int persistent;         // kPersist* bits: raster kernels whose CTAs take cost-ordered items persistently
 };
+// (Tile, segment) items of a segmented 16x16 backward: a launch of few tiles
+// cuts every tile's list into up to kSegMax segments, kSegItems over all tiles.
+constexpr uint32_t kSegItems = 16384, kSegMax = 64;
+
 // Bits of ViewSet::persistent (otherwise one CTA per work item).
 constexpr int kPersistFwd = 1, kPersistBwd = 2;
 

@@ -35,8 +35,10 @@
 // end in a tail of long tiles on a few SMs; views of different sizes and
 // visible counts share one queue. The backward's cost is the number of list
 // entries up to the tile's last contributor: the forward appends each item
-// to the list of its cost's bit length (33 lists), and a backward ticket
-// walks the lists from the longest costs down. A persistent forward orders
+// to the list of its cost's bit length (32 lists), and a backward ticket
+// walks the lists from the longest costs down. A launch of few 16x16 tiles
+// cuts every tile's list into segments, each a backward item of its own, from
+// checkpoints that the forward leaves. A persistent forward orders
 // its items by list length with a single-block counting sort first.
 // Otherwise one CTA per item runs in item order.
 #include <algorithm>
@@ -50,19 +52,13 @@ namespace gsr {
 namespace {
 
 // Pixels per lane. The forward gains nothing from more than 2. The
-// backward of 16x16 tiles runs one warp per tile with 8 pixels per lane
-// (raster_bwd_tile_kernel) when the launch has tiles enough to fill the
-// GPU several times over with one-warp CTAs, so that each Gaussian's warp
-// reduction serves the whole tile; otherwise two warps per tile with 4
-// pixels per lane (raster_bwd_kernel), which keeps twice the warps busy on a
-// small view. The other tile shapes run raster_bwd_kernel with 2.
+// backward of 16x16 tiles runs one warp per tile, or per segment of a tile's
+// list, with 8 pixels per lane (raster_bwd_tile_kernel), so that each
+// Gaussian's warp reduction serves the whole tile; the other tile shapes run
+// raster_bwd_kernel with 2.
 constexpr int kFwdPPL = 2;
 static_assert(4 * kFwdPPL == 8, "forward warp blocks, and so the exported hit bits, are 8x8 pixels");
 constexpr int kBwdPPL = 2;
-constexpr int kBwdPPL16 = 4;
-// One-warp CTA waves (the tile kernel's residency times the SMs) a launch
-// must fill before the 16x16 backward runs one warp per tile.
-constexpr uint32_t kTileKernelWaves = 4;
 // The one-warp backward's batch (entries staged per round, double-buffered)
 // and its resident CTAs per SM: 64 entries take 13 KB of shared memory, so
 // that 16 CTAs fit an SM, the register bound of 16 (at most 128 a thread).
@@ -89,27 +85,30 @@ __device__ __forceinline__ uint32_t find_view(const ViewSet& vs, uint32_t item) 
 
 constexpr uint32_t kNoItem = 0xffffffffu;
 
-constexpr int kCostLists = 33;  // bit lengths 0..32 of a cost
+constexpr int kCostLists = 32;  // bit lengths 0..31 of a cost (a list is shorter than 2^30); one per lane
 
 __device__ __forceinline__ uint32_t cost_bucket(uint32_t cost) { return cost ? 32u - (uint32_t)__clz(cost) : 0u; }
 
-// Per CTA, for the cost lists: each list's length and its first ticket
-// (lists in decreasing cost order). Read once per launch.
+// Per CTA, for the cost lists, entry l the list of the l-th largest costs:
+// its length and its first place in the order. Read once per launch, one load
+// per lane of warp 0 and a warp scan, because a small launch's first items
+// wait for it.
 struct CostListView {
   uint32_t count[kCostLists];
   uint32_t first[kCostLists];
 };
 __device__ __forceinline__ void load_cost_lists(const RasterArgs& a, CostListView* s) {
-  if (!a.persist) return;
-  if (threadIdx.x == 0) {
-    uint32_t run = 0;
-    for (int k = kCostLists - 1; k >= 0; --k) {
-      const uint32_t n = a.b.sched_lcount[k];
-      s->count[k] = n;
-      s->first[k] = run;
-      run += n;
-    }
+  if (!a.persist || threadIdx.x >= 32) return;
+  const uint32_t lane = threadIdx.x;
+  const uint32_t n = a.b.sched_lcount[kCostLists - 1 - lane];
+  uint32_t incl = n;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= (uint32_t)d) incl += t;
   }
+  s->count[lane] = n;
+  s->first[lane] = incl - n;
 }
 
 // The next work item of this CTA (block-uniform; kNoItem when done). In
@@ -131,14 +130,38 @@ __device__ __forceinline__ uint32_t next_item(const RasterArgs& a, uint32_t roun
     return slot < a.vs.total_tiles ? a.b.sched_order[slot] : kNoItem;
   });
 }
+// FIRST (launches whose items fit the resident CTAs a few times over): a CTA's
+// first place is its own index, without a ticket, and warp 0's lanes look
+// through the lists at once, because there an item's start is a good part of
+// its time.
+template <bool FIRST>
 __device__ __forceinline__ uint32_t next_item(const RasterArgs& a, uint32_t round, uint32_t* s_item,
                                               const CostListView* lists) {
-  return take_item(a, round, s_item, [&](uint32_t slot) {
-    for (int k = kCostLists - 1; k >= 0; --k)
-      if (slot - lists->first[k] < lists->count[k])
-        return a.b.sched_lists[(size_t)k * a.b.sched_items_cap + (slot - lists->first[k])];
-    return kNoItem;
-  });
+  if constexpr (!FIRST) {
+    return take_item(a, round, s_item, [&](uint32_t slot) {
+#pragma unroll 1
+      for (int k = 0; k < kCostLists; ++k)
+        if (slot - lists->first[k] < lists->count[k])
+          return a.b.sched_lists[(size_t)(kCostLists - 1 - k) * a.b.sched_items_cap + (slot - lists->first[k])];
+      return kNoItem;
+    });
+  }
+  if (!a.persist) return round == 0 ? blockIdx.x : kNoItem;
+  __syncthreads();
+  if (threadIdx.x == 0) *s_item = kNoItem;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    uint32_t slot = blockIdx.x;
+    if (round > 0) {
+      if (threadIdx.x == 0) slot = gridDim.x + atomicAdd(a.b.sched_ticket, 1u);
+      slot = __shfl_sync(0xffffffffu, slot, 0);
+    }
+    const uint32_t at = slot - lists->first[threadIdx.x];  // wraps past every count below the list's first place
+    if (at < lists->count[threadIdx.x])
+      *s_item = a.b.sched_lists[(size_t)(kCostLists - 1 - threadIdx.x) * a.b.sched_items_cap + at];
+  }
+  __syncthreads();
+  return *s_item;
 }
 
 // One block: the work items of a persistent forward in decreasing order of
@@ -284,6 +307,12 @@ __device__ __forceinline__ float2 blend_exp2(float2 sigma) {
   return make_float2(__uint_as_float(__float_as_uint(p.x) + ex), __uint_as_float(__float_as_uint(p.y) + ey));
 }
 
+// Entries per segment of a list of `len` entries cut into at most k segments:
+// 32 where that covers the list, else 64 (the last segment takes the rest).
+// An item of a latency-bound launch takes about 1000 cycles an entry, so
+// short segments end it sooner; more than 64 would only lengthen its tail.
+__device__ __forceinline__ uint32_t segment_len(uint32_t len, uint32_t k) { return len <= 32u * k ? 32u : 64u; }
+
 // A list entry as the forward stages it. Values that both pixels of a pair
 // take lie twice side by side, so that a load brings them as the register
 // pair a two-wide operation wants.
@@ -313,15 +342,24 @@ constexpr int kFwdThreadsPerSm = 768;
 // on a pixel: a pixel that does not take an entry blends with alpha 0, which
 // leaves its colour and transmittance bit for bit unchanged, and a saturated
 // pixel (transmittance below 1e-4) takes nothing. What bounds it is
-// instruction issue (0.71 of the slots) and, on launches of few tiles, the
-// latency of the longest tile. Against a walk of two entries with a vote and
+// instruction issue and, on launches of few tiles, the latency of the
+// longest tile. Against a walk of two entries with a vote and
 // a branch each, over blocks culled by the footprint's bounding box: 8 views
 // of 1280x720 over 1M Gaussians 1.10 -> 0.83 ms (135M -> 90M warp instructions
 // a view), one view of 320x240 over 74k 0.193 -> 0.104 ms.
-template <int TW, int TH, int BATCH>
-__global__ void __launch_bounds__(TW* TH / 2, kFwdThreadsPerSm / (TW * TH / 2)) raster_fwd_kernel(RasterArgs a) {
+// CKPT: at the end of every segment of the list (segment_len entries) the
+// tile's pixels leave a checkpoint for the segmented backward (see
+// raster_bwd_tile_kernel): the transmittance there and the colour the segment
+// added, turned into the colour of all later segments once the tile is done.
+// The colour is summed per segment on its own, not taken as a difference of
+// running totals, so that what lies far behind keeps its relative accuracy.
+// The next batch's records are then also loaded while the current one is
+// walked, since few warps are there to hide the loads.
+template <int TW, int TH, int BATCH, bool CKPT>
+__global__ void __launch_bounds__(TW* TH / 2, CKPT ? 4 : kFwdThreadsPerSm / (TW * TH / 2)) raster_fwd_kernel(RasterArgs a) {
   constexpr int NT = TW * TH / 2;
   constexpr int NW = NT / 32;
+  constexpr int kSI = (BATCH + NT - 1) / NT;  // entries a thread stages per batch
   static_assert(NW <= 4 && TW % 8 == 0 && TH % 8 == 0, "hit bits of at most four 8x8 blocks");
   __shared__ FwdEntry s_e[BATCH + 1];  // the last one is never taken: it pads the lists
   __shared__ uint8_t s_mask[BATCH];
@@ -358,6 +396,12 @@ __global__ void __launch_bounds__(TW* TH / 2, kFwdThreadsPerSm / (TW * TH / 2)) 
     float2 T = make_float2(in0 ? 1.f : 0.f, in1 ? 1.f : 0.f);
     float2 C0 = f2(0.f), C1 = f2(0.f), C2 = f2(0.f);
     uint32_t last0 = 0, last1 = 0, nc0 = 0, nc1 = 0;
+    // Checkpoints of this tile, segment by segment: half h of thread t's pair
+    // at ck[segment * pixels + h * threads + t].
+    float4* ck = CKPT ? a.b.ckpt + (size_t)item * a.b.seg_k * (TW * TH) + threadIdx.x : nullptr;
+    float2 S0 = f2(0.f), S1 = f2(0.f), S2 = f2(0.f);  // colour added since the last checkpoint
+    uint32_t stored = 0;                              // checkpoints written
+    const uint32_t seg_len = segment_len(s1 - s0, a.b.seg_k);
     struct Raw {
       uint32_t c;
       float4 r0, r1, r2;
@@ -388,21 +432,30 @@ __global__ void __launch_bounds__(TW* TH / 2, kFwdThreadsPerSm / (TW * TH / 2)) 
       E.cidx = r.c;
       s_mask[j] = (uint8_t)reached_blocks<TW, NW>(r.r0.x, r.r0.y, r.r0.z, r.r0.w, r.r1.x, cut, tx0, ty0);
     };
+    Raw next[CKPT ? kSI : 1];  // CKPT: this thread's entries of the next batch
+    auto fetch = [&](uint32_t b0) {
+#pragma unroll
+      for (int i = 0; i < kSI; ++i) {
+        const uint32_t j = threadIdx.x + i * NT;
+        if (j < (uint32_t)BATCH && b0 + j < s1) next[CKPT ? i : 0] = load(b0 + j);
+      }
+    };
+    if (CKPT) fetch(s0);
     for (uint32_t b0 = s0; b0 < s1; b0 += BATCH) {
       const uint32_t nb = min((uint32_t)BATCH, s1 - b0);
-      for (uint32_t j = threadIdx.x; j < nb; j += NT) stage(j, b0 + j, load(b0 + j));
-      __syncthreads();
-      if (!__all_sync(0xffffffffu, T.x < 1e-4f && T.y < 1e-4f)) {
-        // The entries of this warp's block in list order, padded to a multiple
-        // of the unroll.
-        uint32_t cnt = 0;
-        for (uint32_t base = 0; base < nb; base += 32) {
-          const uint32_t j = base + lane;
-          const bool bit = j < nb && ((s_mask[j] >> warp) & 1u);
-          const uint32_t bal = __ballot_sync(0xffffffffu, bit);
-          if (bit) list[cnt + __popc(bal & ((1u << lane) - 1u))] = (uint16_t)(j * sizeof(FwdEntry));
-          cnt += __popc(bal);
+      if (CKPT) {
+#pragma unroll
+        for (int i = 0; i < kSI; ++i) {
+          const uint32_t j = threadIdx.x + i * NT;
+          if (j < nb) stage(j, b0 + j, next[CKPT ? i : 0]);
         }
+      } else {
+        for (uint32_t j = threadIdx.x; j < nb; j += NT) stage(j, b0 + j, load(b0 + j));
+      }
+      __syncthreads();
+      if (CKPT && b0 + BATCH < s1) fetch(b0 + BATCH);
+      // The walk over cnt listed entries, padded to a multiple of the unroll.
+      auto walk = [&](uint32_t cnt) {
         if (lane < kFwdUnroll) list[cnt + lane] = (uint16_t)(BATCH * sizeof(FwdEntry));
         __syncwarp();
         for (uint32_t e = 0; e < cnt; e += kFwdUnroll) {
@@ -437,6 +490,11 @@ __global__ void __launch_bounds__(TW* TH / 2, kFwdThreadsPerSm / (TW * TH / 2)) 
             C0 = fma2(E.r, w, C0);  // blend_accum; the colours were clamped at staging
             C1 = fma2(E.g, w, C1);
             C2 = fma2(E.b, w, C2);
+            if constexpr (CKPT) {
+              S0 = fma2(E.r, w, S0);
+              S1 = fma2(E.g, w, S1);
+              S2 = fma2(E.b, w, S2);
+            }
             T = mul2(T, add2(f2(1.f), neg2(am)));
             if (c0 || c1) E.hit[warp] = 1;
             if (c0) {
@@ -450,7 +508,31 @@ __global__ void __launch_bounds__(TW* TH / 2, kFwdThreadsPerSm / (TW * TH / 2)) 
           }
           if (__all_sync(0xffffffffu, T.x < 1e-4f && T.y < 1e-4f)) break;
         }
+      };
+      // The entries of this warp's block in list order: the whole batch, or
+      // (CKPT) 32 at a time, the shortest segment.
+      uint32_t cnt = 0;
+      const bool live = !__all_sync(0xffffffffu, T.x < 1e-4f && T.y < 1e-4f);
+      for (uint32_t base = 0; (CKPT || live) && base < nb; base += 32) {
+        const uint32_t j = base + lane;
+        const bool bit = j < nb && ((s_mask[j] >> warp) & 1u);
+        const uint32_t bal = __ballot_sync(0xffffffffu, bit);
+        if (bit) list[cnt + __popc(bal & ((1u << lane) - 1u))] = (uint16_t)(j * sizeof(FwdEntry));
+        cnt += __popc(bal);
+        if constexpr (CKPT) {
+          if (cnt && !__all_sync(0xffffffffu, T.x < 1e-4f && T.y < 1e-4f)) walk(cnt);
+          cnt = 0;
+          __syncwarp();  // the list is free again
+          if ((stored + 1) * seg_len == b0 - s0 + base + 32 && stored + 1 < a.b.seg_k) {  // the last one is open-ended
+            float4* c = ck + (size_t)stored * (TW * TH);
+            c[0] = make_float4(T.x, S0.x, S1.x, S2.x);
+            c[NT] = make_float4(T.y, S0.y, S1.y, S2.y);
+            S0 = S1 = S2 = f2(0.f);
+            ++stored;
+          }
+        }
       }
+      if (!CKPT && live) walk(cnt);
       __syncthreads();
       for (uint32_t j = threadIdx.x; j < nb; j += NT) {
         const uint32_t h = *reinterpret_cast<const uint32_t*>(s_e[j].hit);
@@ -458,6 +540,19 @@ __global__ void __launch_bounds__(TW* TH / 2, kFwdThreadsPerSm / (TW * TH / 2)) 
         if (h) vis[s_e[j].cidx] = 1;
       }
       if (__syncthreads_and(T.x < 1e-4f && T.y < 1e-4f)) break;
+    }
+    if constexpr (CKPT) {
+      // Each thread turns its own checkpoints' colours into the sum over the
+      // later segments, from the last one forward.
+      for (int k = (int)stored - 1; k >= 0; --k) {
+        float4* c = ck + (size_t)k * (TW * TH);
+        const float4 u = c[0], w = c[NT];
+        c[0] = make_float4(u.x, S0.x, S1.x, S2.x);
+        c[NT] = make_float4(w.x, S0.y, S1.y, S2.y);
+        S0 = add2(S0, make_float2(u.y, w.y));
+        S1 = add2(S1, make_float2(u.z, w.z));
+        S2 = add2(S2, make_float2(u.w, w.w));
+      }
     }
     float4* out = reinterpret_cast<float4*>(a.out_rgba) + vd.pix_base;
     auto finish = [&](uint32_t row, float Tq, float c0, float c1, float c2, uint32_t last, uint32_t nc) {
@@ -475,11 +570,14 @@ __global__ void __launch_bounds__(TW* TH / 2, kFwdThreadsPerSm / (TW * TH / 2)) 
     const uint32_t ml = __reduce_max_sync(0xffffffffu, max(last0, last1));
     if (lane == 0 && ml) atomicMax(&s_work, ml);
     __syncthreads();
-    if (threadIdx.x == 0) {
-      const uint32_t k = cost_bucket(s_work > s0 ? s_work - s0 : 0u);
-      a.b.sched_lists[(size_t)k * a.b.sched_items_cap + atomicAdd(a.b.sched_lcount + k, 1u)] = item;
-      s_work = 0u;
+    const uint32_t cost = s_work > s0 ? s_work - s0 : 0u;
+    const uint32_t nseg = CKPT ? min(a.b.seg_k, max((cost + seg_len - 1u) / seg_len, 1u)) : 1u;
+    for (uint32_t g = threadIdx.x; g < nseg; g += NT) {  // the tile's backward items, one per segment
+      const uint32_t k = cost_bucket(g + 1 < nseg ? seg_len : cost - g * seg_len);
+      a.b.sched_lists[(size_t)k * a.b.sched_items_cap + atomicAdd(a.b.sched_lcount + k, 1u)] = item * a.b.seg_k + g;
     }
+    __syncthreads();
+    if (threadIdx.x == 0) s_work = 0u;
   }
 }
 
@@ -746,7 +844,7 @@ __global__ void __launch_bounds__(TW* TH / PPL) raster_bwd_kernel(RasterArgs a) 
   __shared__ CostListView s_lists;
   load_cost_lists(a, &s_lists);
   for (uint32_t round = 0;; ++round) {
-    const uint32_t item = next_item(a, round, &s_item, &s_lists);
+    const uint32_t item = next_item<false>(a, round, &s_item, &s_lists);
     if (item == kNoItem) break;
     const uint32_t v = find_view(a.vs, item);
     const ViewDesc& vd = a.vs.views[v];
@@ -942,7 +1040,7 @@ __global__ void __launch_bounds__(TW* TH / PPL) raster_bwd_kernel(RasterArgs a) 
           }
         }
         if (a.det) {
-          reinterpret_cast<float4*>(part + (size_t)(bs + j) * 12)[k] = f;
+          if (any) reinterpret_cast<float4*>(part + (size_t)(bs + j) * 12)[k] = f;
         } else if (f.x != 0.f || f.y != 0.f || f.z != 0.f || f.w != 0.f) {
           atomicAdd(sgrad + (size_t)s_cidx[buf][j] * 3 + k, f);
         }
@@ -955,15 +1053,6 @@ __global__ void __launch_bounds__(TW* TH / PPL) raster_bwd_kernel(RasterArgs a) 
       buf ^= 1;
     }
     asm volatile("cp.async.wait_all;" ::: "memory");  // no copy may outlive the block
-    // Deterministic mode: list entries of this tile that no pixel reached keep
-    // zero partial records.
-    if (a.det) {
-      const uint32_t s1 = ranges[2 * t + 1];
-      for (uint32_t s = smax > s0 ? smax : s0; s + threadIdx.x < s1; s += NT) {
-        float4* p4 = reinterpret_cast<float4*>(part + (size_t)(s + threadIdx.x) * 12);
-        p4[0] = p4[1] = p4[2] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
   }
 }
 
@@ -976,7 +1065,12 @@ __global__ void __launch_bounds__(TW* TH / PPL) raster_bwd_kernel(RasterArgs a) 
 // reaches, and the tile's sum needs no second warp. The pairs of a block
 // column share dx and the terms that depend on it; the sigma-gradient
 // moments are kept per column (S1 = dx0 M0_0 + dx1 M0_1 and so on).
-template <int BATCH, bool REF>
+// SEG: an item is one segment of a tile's list (launches of few tiles, see
+// pick_segments). Its pixels start from the forward's checkpoint at the
+// segment's end: the transmittance there, and the colour behind it, which
+// enters as its dot product with the upstream gradient. The segment's entries
+// are then walked as a whole tile's are.
+template <int BATCH, bool REF, bool SEG>
 __global__ void __launch_bounds__(32, kTileBwdBlocks) raster_bwd_tile_kernel(RasterArgs a) {
   constexpr int NT = 32;
   constexpr int kSI = BATCH / NT;  // entries a lane stages per batch
@@ -994,8 +1088,9 @@ __global__ void __launch_bounds__(32, kTileBwdBlocks) raster_bwd_tile_kernel(Ras
   const int slot = reduce12_slot(lane);                          // the gradient value this lane ends with
   const bool writer = (lane & 1) == 0 && !((lane & 2) && (lane & 4));  // one lane per value
   for (uint32_t round = 0;; ++round) {
-    const uint32_t item = next_item(a, round, &s_item, &s_lists);
-    if (item == kNoItem) break;
+    const uint32_t work = next_item<SEG>(a, round, &s_item, &s_lists);
+    if (work == kNoItem) break;
+    const uint32_t item = SEG ? work / a.b.seg_k : work, seg = SEG ? work % a.b.seg_k : 0u;
     const uint32_t v = find_view(a.vs, item);
     const ViewDesc& vd = a.vs.views[v];
     const uint32_t t = item - vd.tile_base;
@@ -1008,6 +1103,7 @@ __global__ void __launch_bounds__(32, kTileBwdBlocks) raster_bwd_tile_kernel(Ras
                           -((float)(py0 + 12) + 0.5f)};
     const uint32_t* ranges = slice(a.b.ranges, 2 * a.b.Tcap, v);
     const uint32_t s0 = ranges[2 * t];
+    const uint32_t seg_len = SEG ? segment_len(ranges[2 * t + 1] - s0, a.b.seg_k) : 0u;
     const uint32_t* vals = isect_index_src(a.b, v);
     const uint32_t vmask = isect_index_mask(a.b);
     const float4* rec = slice(a.b.rec, a.b.Vcap * 3, v);
@@ -1025,7 +1121,24 @@ __global__ void __launch_bounds__(32, kTileBwdBlocks) raster_bwd_tile_kernel(Ras
       s_v[q][2][lane] = pp[q].vb;
     }
     const uint32_t smax = __reduce_max_sync(0xffffffffu, mylast);
-    auto batch_lo = [&](uint32_t e) { return (e - s0 > (uint32_t)BATCH) ? e - BATCH : s0; };
+    // This segment's entries [lo, hi); the last segment ends at the tile's
+    // last contributor and starts from the pixels' final state, the others
+    // from their checkpoint.
+    const uint32_t lo = SEG ? s0 + seg * seg_len : s0;
+    if (SEG && seg > 0 && lo >= smax) continue;  // grid schedule: past the tile's segments
+    const bool final_seg = !SEG || seg + 1 == a.b.seg_k || smax <= lo + seg_len;
+    const uint32_t hi = final_seg ? smax : lo + seg_len;
+    if (!final_seg) {
+      const float4* ck = a.b.ckpt + (size_t)work * 256 + lane;
+  #pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 u = ck[q * 32], w = ck[128 + q * 32];
+        pp[q].T = make_float2(u.x, w.x);
+        pp[q].SK = add2(pp[q].SK, fma2(make_float2(u.w, w.w), pp[q].vb,
+                                       fma2(make_float2(u.z, w.z), pp[q].vg, mul2(make_float2(u.y, w.y), pp[q].vr))));
+      }
+    }
+    auto batch_lo = [&](uint32_t e) { return (e - lo > (uint32_t)BATCH) ? e - BATCH : lo; };
     uint32_t pc[kSI], ph[kSI];
     auto fetch = [&](uint32_t lo, uint32_t hi) {
   #pragma unroll
@@ -1053,22 +1166,22 @@ __global__ void __launch_bounds__(32, kTileBwdBlocks) raster_bwd_tile_kernel(Ras
       }
       cp_async_commit();
     };
-    uint32_t be = smax, bs = be > s0 ? batch_lo(be) : s0;
-    if (be > s0) {
+    uint32_t be = hi, bs = be > lo ? batch_lo(be) : lo;
+    if (be > lo) {
       fetch(bs, be);
       issue(bs, be, 0);
     }
-    uint32_t nbe = bs, nbs = nbe > s0 ? batch_lo(nbe) : s0;
-    if (nbe > s0) fetch(nbs, nbe);
+    uint32_t nbe = bs, nbs = nbe > lo ? batch_lo(nbe) : lo;
+    if (nbe > lo) fetch(nbs, nbe);
     int buf = 0;
-    while (be > s0) {
+    while (be > lo) {
       const uint32_t nb = be - bs;
-      if (nbe > s0)
+      if (nbe > lo)
         issue(nbs, nbe, buf ^ 1);
       else
         cp_async_commit();
-      const uint32_t n2e = nbs, n2s = n2e > s0 ? batch_lo(n2e) : s0;
-      if (n2e > s0) fetch(n2s, n2e);
+      const uint32_t n2e = nbs, n2s = n2e > lo ? batch_lo(n2e) : lo;
+      if (n2e > lo) fetch(n2s, n2e);
       cp_async_wait1();  // this lane's copies of the current batch have landed
       __syncthreads();   // and every lane's
       const int cnt = build_list(s_mask[buf], nb, 0xfu, lane, s_list);
@@ -1164,7 +1277,7 @@ __global__ void __launch_bounds__(32, kTileBwdBlocks) raster_bwd_tile_kernel(Ras
           }
         }
         if (a.det) {
-          reinterpret_cast<float4*>(part + (size_t)(bs + j) * 12)[k] = f;
+          if (s_mask[buf][j]) reinterpret_cast<float4*>(part + (size_t)(bs + j) * 12)[k] = f;
         } else if (f.x != 0.f || f.y != 0.f || f.z != 0.f || f.w != 0.f) {
           atomicAdd(sgrad + (size_t)s_cidx[buf][j] * 3 + k, f);
         }
@@ -1177,14 +1290,19 @@ __global__ void __launch_bounds__(32, kTileBwdBlocks) raster_bwd_tile_kernel(Ras
       buf ^= 1;
     }
     asm volatile("cp.async.wait_all;" ::: "memory");  // no copy may outlive the block
-    if (a.det) {
-      const uint32_t s1 = ranges[2 * t + 1];
-      for (uint32_t s = smax > s0 ? smax : s0; s + lane < s1; s += NT) {
-        float4* p4 = reinterpret_cast<float4*>(part + (size_t)(s + lane) * 12);
-        p4[0] = p4[1] = p4[2] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
   }
+}
+
+// Deterministic mode: zero partial sums for every intersection; the backward
+// then writes those of the entries that some pixel took. Most list entries
+// lie behind saturated pixels, and a warp per tile clearing its own list's
+// rest took up to half of the kernel; this is a plain sweep at HBM rate.
+__global__ void __launch_bounds__(256) zero_parts_kernel(FwdBufs b) {
+  const uint32_t v = blockIdx.y;
+  const uint64_t n = (uint64_t)b.vcount[v * 4 + 1] * 3;
+  float4* part = reinterpret_cast<float4*>(b.sgrad_part + (size_t)b.Icap * 12 * v);
+  for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (uint64_t)gridDim.x * 256)
+    part[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // Gaussians per shared-memory batch: 0 selects the tuned defaults (128 in
@@ -1217,8 +1335,8 @@ template <void (*Kernel)(RasterArgs)> int resident_per_sm(int threads) {
 }
 
 template <void (*Kernel)(RasterArgs)>
-cudaError_t launch_items(int threads, const RasterArgs& a, int num_sms, cudaStream_t st) {
-  uint32_t grid = a.vs.total_tiles;
+cudaError_t launch_items(int threads, const RasterArgs& a, uint32_t items, int num_sms, cudaStream_t st) {
+  uint32_t grid = items;
   if (a.persist)
     grid = std::min<uint32_t>(grid, (uint32_t)resident_per_sm<Kernel>(threads) * (uint32_t)std::max(num_sms, 1));
   if (grid == 0) return cudaSuccess;  // a warm-up call (no items)
@@ -1226,47 +1344,73 @@ cudaError_t launch_items(int threads, const RasterArgs& a, int num_sms, cudaStre
   return cudaGetLastError();
 }
 
+template <int TW, int TH, int BATCH, bool CKPT>
+cudaError_t launch_fwd_batch(const RasterArgs& a, int num_sms, cudaStream_t st) {
+  return launch_items<raster_fwd_kernel<TW, TH, BATCH, CKPT>>(TW * TH / 2, a, a.vs.total_tiles, num_sms, st);
+}
 template <int TW, int TH>
 cudaError_t launch_fwd_shape(const RasterArgs& a, uint32_t batch, int num_sms, cudaStream_t st) {
-  constexpr int NT = TW * TH / 2;
   switch (pick_batch(batch, 128)) {
-    case 64: return launch_items<raster_fwd_kernel<TW, TH, 64>>(NT, a, num_sms, st);
-    case 128: return launch_items<raster_fwd_kernel<TW, TH, 128>>(NT, a, num_sms, st);
-    default: return launch_items<raster_fwd_kernel<TW, TH, 256>>(NT, a, num_sms, st);
+    case 64: return launch_fwd_batch<TW, TH, 64, false>(a, num_sms, st);
+    case 128: return launch_fwd_batch<TW, TH, 128, false>(a, num_sms, st);
+    default: return launch_fwd_batch<TW, TH, 256, false>(a, num_sms, st);
+  }
+}
+// 16x16 tiles: with checkpoints when the backward is segmented.
+cudaError_t launch_fwd_16(const RasterArgs& a, uint32_t batch, int num_sms, cudaStream_t st) {
+  if (a.b.seg_k == 1) return launch_fwd_shape<16, 16>(a, batch, num_sms, st);
+  switch (pick_batch(batch, 64)) {
+    case 64: return launch_fwd_batch<16, 16, 64, true>(a, num_sms, st);
+    case 128: return launch_fwd_batch<16, 16, 128, true>(a, num_sms, st);
+    default: return launch_fwd_batch<16, 16, 256, true>(a, num_sms, st);
   }
 }
 template <int TW, int TH, int PPL, bool REF>
 cudaError_t launch_bwd_mode(const RasterArgs& a, uint32_t batch, int num_sms, cudaStream_t st) {
   constexpr int NT = TW * TH / PPL;
   constexpr int kMaxBatch = NT / 32 >= 2 ? 128 : 256;
+  const uint32_t items = a.vs.total_tiles;
   int b = pick_batch(batch, 64);
   if (b > kMaxBatch) b = kMaxBatch;
   switch (b) {
-    case 64: return launch_items<raster_bwd_kernel<TW, TH, PPL, 64, REF>>(NT, a, num_sms, st);
-    case 128: return launch_items<raster_bwd_kernel<TW, TH, PPL, 128, REF>>(NT, a, num_sms, st);
+    case 64: return launch_items<raster_bwd_kernel<TW, TH, PPL, 64, REF>>(NT, a, items, num_sms, st);
+    case 128: return launch_items<raster_bwd_kernel<TW, TH, PPL, 128, REF>>(NT, a, items, num_sms, st);
     default:
-      return launch_items<raster_bwd_kernel<TW, TH, PPL, (kMaxBatch > 128 ? 256 : 128), REF>>(NT, a, num_sms, st);
+      return launch_items<raster_bwd_kernel<TW, TH, PPL, (kMaxBatch > 128 ? 256 : 128), REF>>(NT, a, items, num_sms,
+                                                                                               st);
   }
-}
-// The 16x16 backward stages 64 entries per batch whatever the forward's
-// batch: 13 KB of shared memory and at most 128 registers per one-warp CTA
-// let 16 CTAs share an SM (a 128-entry batch would fit 9).
-template <bool REF>
-cudaError_t launch_bwd_tile16(const RasterArgs& a, int num_sms, cudaStream_t st) {
-  return launch_items<raster_bwd_tile_kernel<kTileBwdBatch, REF>>(32, a, num_sms, st);
 }
 template <int TW, int TH, int PPL>
 cudaError_t launch_bwd_shape(const RasterArgs& a, uint32_t batch, int num_sms, cudaStream_t st) {
   return a.ref_mode ? launch_bwd_mode<TW, TH, PPL, true>(a, batch, num_sms, st)
                     : launch_bwd_mode<TW, TH, PPL, false>(a, batch, num_sms, st);
 }
-// 16x16 tiles: one warp per tile on large launches, two otherwise.
-cudaError_t launch_bwd_16(const RasterArgs& a, uint32_t batch, int num_sms, cudaStream_t st) {
-  const uint32_t wave =
-      (uint32_t)resident_per_sm<raster_bwd_tile_kernel<kTileBwdBatch, false>>(32) * (uint32_t)std::max(num_sms, 1);
-  if (a.vs.total_tiles >= kTileKernelWaves * wave || a.vs.total_tiles == 0)
-    return a.ref_mode ? launch_bwd_tile16<true>(a, num_sms, st) : launch_bwd_tile16<false>(a, num_sms, st);
-  return launch_bwd_shape<16, 16, kBwdPPL16>(a, batch, num_sms, st);
+// 16x16 tiles: one warp per (tile, segment). It stages 64 entries per batch
+// whatever the forward's batch: 13 KB of shared memory and at most 128
+// registers per one-warp CTA let 16 CTAs share an SM (a 128-entry batch would
+// fit 9).
+template <bool REF>
+cudaError_t launch_bwd_tile16(const RasterArgs& a, int num_sms, cudaStream_t st) {
+  const uint32_t items = a.vs.total_tiles * a.b.seg_k;
+  return a.b.seg_k > 1 ? launch_items<raster_bwd_tile_kernel<kTileBwdBatch, REF, true>>(32, a, items, num_sms, st)
+                       : launch_items<raster_bwd_tile_kernel<kTileBwdBatch, REF, false>>(32, a, items, num_sms, st);
+}
+cudaError_t launch_bwd_16(const RasterArgs& a, int num_sms, cudaStream_t st) {
+  return a.ref_mode ? launch_bwd_tile16<true>(a, num_sms, st) : launch_bwd_tile16<false>(a, num_sms, st);
+}
+
+// Segments a tile's list is cut into for the backward of this launch (1: none).
+// A launch of few tiles waits for its longest list, one entry after another;
+// segments spread it over the idle SMs, for a forward that writes a checkpoint
+// per segment. Forward plus backward, without and with: 256 tiles (16k
+// Gaussians) 0.295 -> 0.105 ms, 300 tiles (74k) 0.465 -> 0.181, 1200 tiles
+// (200k) 0.303 -> 0.218, 3600 tiles (500k, 4 segments) 0.377 -> 0.373. With 2
+// segments each it costs more than it gives: 5800 tiles 0.650 -> 0.661, 8160
+// tiles 0.702 -> 0.733. So at least 4, that is at most 4096 tiles.
+uint32_t pick_segments(const ViewSet& vs) {
+  if (vs.tile_w != 16 || vs.tile_h != 16 || vs.total_tiles == 0) return 1;
+  const uint32_t k = std::min(kSegMax, kSegItems / vs.total_tiles);
+  return k < 4 ? 1 : k;
 }
 
 }  // namespace
@@ -1278,9 +1422,12 @@ void raster_warm_up(uint32_t tile_w, uint32_t tile_h, uint32_t batch, int num_sm
   for (int ref = 0; ref < 2; ++ref) {
     a.ref_mode = ref;
     if (tile_w == 16 && tile_h == 16) {
-      (void)launch_fwd_shape<16, 16>(a, batch, num_sms, nullptr);
-      (void)launch_bwd_16(a, batch, num_sms, nullptr);
-      (void)launch_bwd_shape<16, 16, kBwdPPL16>(a, batch, num_sms, nullptr);
+      a.b.seg_k = 1;
+      (void)launch_fwd_16(a, batch, num_sms, nullptr);
+      (void)launch_bwd_16(a, num_sms, nullptr);
+      a.b.seg_k = 2;
+      (void)launch_fwd_16(a, batch, num_sms, nullptr);
+      (void)launch_bwd_16(a, num_sms, nullptr);
     } else if (tile_w == 8 && tile_h == 8) {
       (void)launch_fwd_shape<8, 8>(a, batch, num_sms, nullptr);
       (void)launch_bwd_shape<8, 8, kBwdPPL>(a, batch, num_sms, nullptr);
@@ -1293,6 +1440,7 @@ void raster_warm_up(uint32_t tile_w, uint32_t tile_h, uint32_t batch, int num_sm
 
 cudaError_t launch_raster_fwd(const ViewSet& vs, FwdBufs& b, const float* bg, float* out_rgba, const Scratch& s,
                               cudaStream_t st) {
+  b.seg_k = pick_segments(vs);
   RasterArgs a{};
   a.vs = vs;
   a.b = b;
@@ -1312,7 +1460,7 @@ cudaError_t launch_raster_fwd(const ViewSet& vs, FwdBufs& b, const float* bg, fl
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  if (vs.tile_w == 16 && vs.tile_h == 16) return launch_fwd_shape<16, 16>(a, vs.batch, s.num_sms, st);
+  if (vs.tile_w == 16 && vs.tile_h == 16) return launch_fwd_16(a, vs.batch, s.num_sms, st);
   if (vs.tile_w == 8 && vs.tile_h == 8) return launch_fwd_shape<8, 8>(a, vs.batch, s.num_sms, st);
   if (vs.tile_w == 32 && vs.tile_h == 8) return launch_fwd_shape<32, 8>(a, vs.batch, s.num_sms, st);
   return cudaErrorInvalidValue;
@@ -1329,7 +1477,11 @@ cudaError_t launch_raster_bwd(const ViewSet& vs, FwdBufs& b, const float* bg, co
   a.v_rgba = v_rgba;
   a.ref_mode = ref_mode;
   a.det = deterministic;
-  if (!deterministic) {
+  if (deterministic) {
+    zero_parts_kernel<<<dim3(std::max(1, s.num_sms * 8 / (int)vs.n_views), vs.n_views), 256, 0, st>>>(b);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  } else {
     cudaError_t e = cudaMemsetAsync(b.sgrad, 0, sizeof(float4) * 3 * b.Vcap * vs.n_views, st);
     if (e != cudaSuccess) return e;
   }
@@ -1339,7 +1491,7 @@ cudaError_t launch_raster_bwd(const ViewSet& vs, FwdBufs& b, const float* bg, co
     cudaError_t e = cudaMemsetAsync(b.sched_ticket, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
   }
-  if (vs.tile_w == 16 && vs.tile_h == 16) return launch_bwd_16(a, vs.batch, s.num_sms, st);
+  if (vs.tile_w == 16 && vs.tile_h == 16) return launch_bwd_16(a, s.num_sms, st);
   if (vs.tile_w == 8 && vs.tile_h == 8) return launch_bwd_shape<8, 8, kBwdPPL>(a, vs.batch, s.num_sms, st);
   if (vs.tile_w == 32 && vs.tile_h == 8) return launch_bwd_shape<32, 8, kBwdPPL>(a, vs.batch, s.num_sms, st);
   return cudaErrorInvalidValue;
