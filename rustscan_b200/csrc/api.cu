@@ -194,6 +194,7 @@ gsr_status allocate(gsr_ctx* c) {
   if (!ok) return fail(c, GSR_ERR_OOM, "device allocation failed (reduce max_splats/max_isects/max_pixels)");
   c->s.lb_states_words = c->states_words;
   c->s.num_sms = c->num_sms;
+  c->s.cluster_sort = cluster_sort_available();
   // Zero the look-back states (epoch 0 never matches a launch), the control
   // block and the status words.
   if (cudaMemset(c->s.lb_states, 0, sizeof(unsigned long long) * c->states_words) != cudaSuccess ||
@@ -309,8 +310,11 @@ gsr_status forward_impl(gsr_ctx* c, const gsr_splats* sp, const gsr_camera* cams
   prof_mark(c, kStProject, st);
   GSR_CUDA(c, launch_project(sd, vs, c->cfg.cov_blur, c->cfg.fp64_conic, b, c->s, st));
   prof_mark(c, kStDepthSort, st);
-  GSR_CUDA(c, radix_sort_pairs(b.depth_key, nullptr, b.depth_sorted, b.perm, b.key_tmp, b.val_tmp, b.Vcap, n_views,
-                               b.vcount, 4, 0, b.Vcap, 31, c->s, st));
+  // Few Gaussians: one cluster per view sorts and scans at once, below.
+  const bool one_launch = order_fits_cluster(sp->n, n_views, c->s);
+  if (!one_launch)
+    GSR_CUDA(c, radix_sort_pairs(b.depth_key, nullptr, b.depth_sorted, b.perm, b.key_tmp, b.val_tmp, b.Vcap, n_views,
+                                 b.vcount, 4, 0, b.Vcap, 31, c->s, st));
   // Up to kHistMaxTiles tiles a view, emission also counts intersections
   // per tile: the tile ranges and the tile sort's digit histograms follow
   // from those counts (no histogram pass, no ranges pass).
@@ -328,7 +332,10 @@ gsr_status forward_impl(gsr_ctx* c, const gsr_splats* sp, const gsr_camera* cams
   b.slots = tile_counts && !c->cfg.deterministic && vs.max_tiles < (1u << tbits);
   prof_mark(c, kStOffsets, st);
   if (!b.slots) GSR_CUDA(c, launch_count(vs, b, c->s, st));
-  GSR_CUDA(c, launch_offsets(vs, b, c->s, st));
+  if (one_launch)
+    GSR_CUDA(c, launch_order_offsets(vs, sp->n, b, c->s, st));
+  else
+    GSR_CUDA(c, launch_offsets(vs, b, c->s, st));
   prof_mark(c, kStEmit, st);
   // In the slot layout the tile sort drops the failing tiles' sentinel keys
   // in its first pass when its digits leave a spare digit value (below 8

@@ -103,6 +103,7 @@ struct Scratch {
   LookbackCtl* ctl;
   DevStatus* status;
   int num_sms;
+  bool cluster_sort;              // the device holds the clusters of launch_order_offsets
 };
 
 // Gaussians per projection block (visibility, per-block counts, records).
@@ -165,6 +166,13 @@ cudaError_t inclusive_scan_u32_scratch(const uint32_t* in, uint32_t* out, uint32
                                        uint64_t states_words, LookbackCtl* ctl, DevStatus* status, int num_sms,
                                        cudaStream_t st);
 
+// Depth order and offsets of views of few Gaussians in one launch (perm,
+// offset, vcount[1..2]): what radix_sort_pairs on the depth keys and
+// launch_offsets give. For n Gaussians and a number of views that
+// order_fits_cluster accepts.
+bool cluster_sort_available();
+bool order_fits_cluster(uint32_t n, uint32_t views, const Scratch& s);
+cudaError_t launch_order_offsets(const ViewSet& vs, uint32_t n, FwdBufs& b, const Scratch& s, cudaStream_t st);
 // Per view: offset[r] = exclusive scan of count[perm[r]], sets vcount[1..2].
 cudaError_t launch_offsets(const ViewSet& vs, FwdBufs& b, const Scratch& s, cudaStream_t st);
 

@@ -21,6 +21,8 @@
 // when both fit in 32 bits).
 #include <algorithm>
 
+#include <cooperative_groups.h>
+
 #include "gsr_kernels.h"
 
 namespace gsr {
@@ -305,6 +307,268 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(ScanArgs a) {
   epoch_end(a.ctl, epoch);
 }
 
+// ---------------------------------------------------------------------------
+// Depth order and intersection offsets of a small view in one launch: a
+// cluster of 16 CTAs per view holds the view's (key, index) pairs in its
+// shared memory, a chunk of consecutive positions per CTA, and runs every
+// radix pass and the offset scan there. Per pass each warp ranks its pairs
+// stably (as sort_pass_kernel does), the CTAs send their digit counts to one
+// another, and every pair is stored straight to its place in the CTA that
+// owns it. Two cluster barriers per pass take the place of a launch and a
+// look-back. What bounds it, in cycles of one SM: about 1500 per round of 1024
+// pairs to rank, 1300 to send them (single 8-byte stores), 2000 per barrier.
+// ---------------------------------------------------------------------------
+constexpr int kClusterThreads = 1024;
+constexpr int kClusterWarps = kClusterThreads / 32;
+constexpr int kClusterDigits = 512;  // of at most 9 bits
+// Up to 13 pairs per thread of 16 CTAs, and for more than 4 views (the GPU
+// holds about so many of these clusters at a time) few enough pairs that the
+// later waves stay cheap. Depth order and offsets by the radix passes and by
+// the cluster, in us: one view of 14k visible Gaussians 85 and 34, of 55k 93
+// and 44, of 149k 102 and 81, of 179k 106 and 103; 8 views of 55k 106 and 77,
+// of 97k 116 and 107, of 149k 143 and 153; 16 views of 55k 118 and 119.
+constexpr uint32_t kClusterMaxKeys = 16u * kClusterThreads * 13u;
+constexpr uint64_t kClusterMaxWaveKeys = 300000;
+
+struct ClusterSortArgs {
+  const uint32_t* key;    // [V] depth bits (31 of them order)
+  const uint32_t* count;  // [V] intersections per compact index
+  uint32_t* perm;         // [V] compact index per depth rank
+  uint32_t* offset;       // [V] exclusive scan of count[perm]
+  uint64_t stride;        // elements per view
+  uint32_t* vcount;       // [view][4]: visible, intersections (clamped), intersections required, pad
+  uint64_t cap_total;
+  DevStatus* status;
+};
+
+template <int C, int IT> struct ClusterSortSmem {
+  uint2 pair[IT * kClusterThreads];
+  uint16_t whist[kClusterWarps][kClusterDigits];  // per warp: digit counts, then starts
+  uint32_t counts[C][kClusterDigits];             // every CTA's digit counts of the pass
+  uint32_t base[kClusterDigits];
+  uint32_t scan[32];
+  uint32_t red[2][32];
+  uint2 range[C];                                 // every CTA's smallest and largest key
+  uint32_t totals[C];
+};
+
+// C CTAs per cluster, at most IT pairs per thread.
+template <int C, int IT>
+__global__ void __launch_bounds__(kClusterThreads, 1) cluster_sort_kernel(ClusterSortArgs a) {
+  namespace cg = cooperative_groups;
+  extern __shared__ uint4 smem_cs[];
+  ClusterSortSmem<C, IT>& S = *reinterpret_cast<ClusterSortSmem<C, IT>*>(smem_cs);
+  cg::cluster_group cluster = cg::this_cluster();
+  const uint32_t rank = cluster.block_rank(), v = blockIdx.y;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t V = a.vcount[v * 4 + 0];
+  // Pairs per thread (uniform over the cluster) and per CTA; the division of
+  // a position by the chunk is exact for positions below 2^19.
+  const uint32_t it = max((V + C * kClusterThreads - 1) / (C * kClusterThreads), 1u);
+  const uint32_t chunk = it * kClusterThreads;
+  const uint32_t magic = (65536u + it - 1u) / it;
+  const uint32_t first = rank * chunk;
+  const uint32_t mine = V > first ? min(V - first, chunk) : 0u;
+  const uint32_t* key = a.key + a.stride * v;
+  uint2 kv[IT];
+  const uint32_t at0 = warp * 32u * it + lane;  // this thread's pairs: at0 + 32 i
+  uint32_t lo = 0xffffffffu, hi = 0u;
+#pragma unroll
+  for (int i = 0; i < IT; ++i) {
+    const uint32_t j = at0 + 32u * i;
+    if ((uint32_t)i < it && j < mine) {
+      kv[i] = make_uint2(key[first + j] & 0x7fffffffu, first + j);
+      lo = min(lo, kv[i].x);
+      hi = max(hi, kv[i].x);
+    }
+  }
+  // The keys' range over the view: their distances from the smallest order
+  // them as well and take fewer bits (27 hold depths of a ratio of 65536, in
+  // three passes of 9).
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (lane == 0) {
+    S.red[0][warp] = lo;
+    S.red[1][warp] = hi;
+  }
+  __syncthreads();
+  lo = __reduce_min_sync(0xffffffffu, S.red[0][lane]);
+  hi = __reduce_max_sync(0xffffffffu, S.red[1][lane]);
+  if (tid < (uint32_t)C) *cluster.map_shared_rank(&S.range[rank], tid) = make_uint2(lo, hi);
+  cluster.sync();
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    lo = min(lo, S.range[c].x);
+    hi = max(hi, S.range[c].y);
+  }
+  const uint32_t bits = hi > lo ? 32u - (uint32_t)__clz(hi - lo) : 1u;
+  const uint32_t passes = bits <= 27u ? 3u : 4u;
+  const uint32_t dbits = (bits + passes - 1u) / passes;
+  const uint32_t digits = 1u << dbits, dmask = digits - 1u;
+#pragma unroll
+  for (int i = 0; i < IT; ++i) kv[i].x -= lo;
+  for (uint32_t shift = 0; shift < bits; shift += dbits) {
+    for (uint32_t d = lane; d < digits; d += 32u) S.whist[warp][d] = 0;
+    __syncwarp();
+    // Stable rank within the warp: rounds in order, lanes in order.
+    uint32_t ranks[(IT + 1) / 2];  // two 16-bit ranks a word
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      uint32_t r = 0;
+      if ((uint32_t)i < it) {
+        const bool ok = at0 + 32u * i < mine;
+        const uint32_t d = ok ? (kv[i].x >> shift) & dmask : 0u;
+        uint32_t peers = __ballot_sync(0xffffffffu, ok);
+#pragma unroll
+        for (int bit = 0; bit < 9; ++bit) {
+          const bool set = (d >> bit) & 1u;
+          const uint32_t bb = __ballot_sync(0xffffffffu, set);
+          peers &= set ? bb : ~bb;
+        }
+        const uint32_t below = peers & ((1u << lane) - 1u);
+        const uint32_t b = ok ? S.whist[warp][d] : 0u;
+        __syncwarp();
+        if (ok && below == 0) S.whist[warp][d] = (uint16_t)(b + __popc(peers));
+        __syncwarp();
+        r = b + __popc(below);
+      }
+      if (i & 1)
+        ranks[i / 2] |= r << 16;
+      else
+        ranks[i / 2] = r;
+    }
+    __syncthreads();
+    // One thread per digit: warp starts, and the CTA's count to every CTA.
+    uint32_t sum = 0;
+    if (tid < digits) {
+#pragma unroll 16
+      for (int w = 0; w < kClusterWarps; ++w) {
+        const uint32_t t = S.whist[w][tid];
+        S.whist[w][tid] = (uint16_t)sum;
+        sum += t;
+      }
+#pragma unroll
+      for (int c = 0; c < C; ++c) *cluster.map_shared_rank(&S.counts[rank][tid], c) = sum;
+    }
+    cluster.sync();  // the counts have arrived, and every CTA's pairs are in registers
+    uint32_t total = 0, before = 0;
+    if (tid < digits) {
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const uint32_t t = S.counts[c][tid];
+        before += (uint32_t)c < rank ? t : 0u;
+        total += t;
+      }
+    }
+    uint32_t all;
+    const uint32_t start = block_exclusive_scan(total, S.scan, &all);
+    if (tid < digits) S.base[tid] = start + before;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      if ((uint32_t)i < it && at0 + 32u * i < mine) {
+        const uint32_t d = (kv[i].x >> shift) & dmask;
+        const uint32_t pos = S.base[d] + S.whist[warp][d] + ((ranks[i / 2] >> (16 * (i & 1))) & 0xffffu);
+        const uint32_t to = ((pos >> 10) * magic) >> 16;
+        *cluster.map_shared_rank(&S.pair[pos - to * chunk], to) = kv[i];
+      }
+    }
+    cluster.sync();  // the pairs have arrived
+#pragma unroll
+    for (int i = 0; i < IT; ++i) {
+      const uint32_t j = at0 + 32u * i;
+      if ((uint32_t)i < it && j < mine) kv[i] = S.pair[j];
+    }
+  }
+  // Depth order out, and the exclusive scan of the counts along it: a warp's
+  // pairs are consecutive, rounds in order.
+  const uint32_t* count = a.count + a.stride * v;
+  uint32_t* perm = a.perm + a.stride * v;
+  uint32_t* offset = a.offset + a.stride * v;
+#pragma unroll
+  for (int i = 0; i < IT; ++i) {
+    const uint32_t j = at0 + 32u * i;
+    const bool ok = (uint32_t)i < it && j < mine;
+    if (ok) perm[first + j] = kv[i].y;
+    kv[i].x = ok ? count[kv[i].y] : 0u;
+  }
+  uint32_t run = 0;
+#pragma unroll
+  for (int i = 0; i < IT; ++i) {
+    if ((uint32_t)i < it) {
+      uint32_t x = kv[i].x;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= (uint32_t)o) x += y;
+      }
+      kv[i].x = run + x - kv[i].x;  // before this pair, within the warp
+      run += __shfl_sync(0xffffffffu, x, 31);
+    }
+  }
+  uint32_t all;
+  const uint32_t incl = block_exclusive_scan(lane == 31u ? run : 0u, S.scan, &all);
+  const uint32_t wstart = __shfl_sync(0xffffffffu, incl, 0);  // the warps before this one
+  if (tid < (uint32_t)C) *cluster.map_shared_rank(&S.totals[rank], tid) = all;
+  cluster.sync();  // also the last access to another CTA's memory
+  uint64_t total = 0;
+  uint32_t before = 0;
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    if ((uint32_t)c < rank) before += S.totals[c];
+    total += S.totals[c];
+  }
+#pragma unroll
+  for (int i = 0; i < IT; ++i) {
+    const uint32_t j = at0 + 32u * i;
+    if ((uint32_t)i < it && j < mine) offset[first + j] = before + wstart + kv[i].x;
+  }
+  if (rank == 0 && tid == 0) {
+    a.vcount[v * 4 + 1] = (uint32_t)(total < a.cap_total ? total : a.cap_total);
+    a.vcount[v * 4 + 2] = (uint32_t)total;
+    if (total > a.cap_total) {
+      atomicExch(&a.status->overflow, 1u);
+      atomicMax(&a.status->required, (unsigned long long)total);
+    }
+  }
+}
+
+// Launches the kernel or, with only_query, asks whether the device can hold
+// such a cluster.
+template <int C, int IT>
+cudaError_t cluster_sort_launch(const ClusterSortArgs& a, uint32_t views, cudaStream_t st, bool only_query) {
+  constexpr int bytes = (int)sizeof(ClusterSortSmem<C, IT>);
+  auto* kernel = cluster_sort_kernel<C, IT>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && C > 8) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return e;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = C;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(C, views);
+  cfg.blockDim = dim3(kClusterThreads);
+  cfg.dynamicSmemBytes = bytes;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (only_query) {
+    int n = 0;
+    e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+    return e != cudaSuccess ? e : (n > 0 ? cudaSuccess : cudaErrorInvalidConfiguration);
+  }
+  return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+cudaError_t cluster_sort_pick(uint32_t n, const ClusterSortArgs& a, uint32_t views, cudaStream_t st, bool only_query) {
+  const uint32_t k = (n + kClusterThreads - 1) / kClusterThreads;
+  if (k <= 16 * 2) return cluster_sort_launch<16, 2>(a, views, st, only_query);
+  if (k <= 16 * 5) return cluster_sort_launch<16, 5>(a, views, st, only_query);
+  if (k <= 16 * 8) return cluster_sort_launch<16, 8>(a, views, st, only_query);
+  return cluster_sort_launch<16, 13>(a, views, st, only_query);
+}
+
 int persistent_blocks(int num_sms, uint32_t segments, int per_sm) {
   const int total = num_sms * per_sm;
   const int per = total / (int)(segments ? segments : 1);
@@ -420,6 +684,31 @@ cudaError_t inclusive_scan_u32_scratch(const uint32_t* in, uint32_t* out, uint32
   a.status = status;
   scan_kernel<<<dim3(persistent_blocks(num_sms, 1, 4), 1), kScanThreads, 0, st>>>(a);
   return cudaGetLastError();
+}
+
+bool cluster_sort_available() {
+  bool ok = true;
+  for (uint32_t it : {2u, 5u, 8u, 13u})
+    ok = ok && cluster_sort_pick(it * 16u * kClusterThreads, ClusterSortArgs{}, 1, nullptr, true) == cudaSuccess;
+  (void)cudaGetLastError();
+  return ok;
+}
+
+bool order_fits_cluster(uint32_t n, uint32_t views, const Scratch& s) {
+  return s.cluster_sort && n <= kClusterMaxKeys && (uint64_t)n * ((views + 3) / 4) <= kClusterMaxWaveKeys;
+}
+
+cudaError_t launch_order_offsets(const ViewSet& vs, uint32_t n, FwdBufs& b, const Scratch& s, cudaStream_t st) {
+  ClusterSortArgs a{};
+  a.key = b.depth_key;
+  a.count = b.count;
+  a.perm = b.perm;
+  a.offset = b.offset;
+  a.stride = b.Vcap;
+  a.vcount = b.vcount;
+  a.cap_total = b.Icap;
+  a.status = s.status;
+  return cluster_sort_pick(n, a, vs.n_views, st, false);
 }
 
 cudaError_t launch_offsets(const ViewSet& vs, FwdBufs& b, const Scratch& s, cudaStream_t st) {
