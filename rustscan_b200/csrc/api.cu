@@ -194,7 +194,7 @@ gsr_status allocate(gsr_ctx* c) {
   if (!ok) return fail(c, GSR_ERR_OOM, "device allocation failed (reduce max_splats/max_isects/max_pixels)");
   c->s.lb_states_words = c->states_words;
   c->s.num_sms = c->num_sms;
-  c->s.cluster_sort = cluster_sort_available();
+  c->s.cluster_sort = cluster_sort_available(c->device);
   // Zero the look-back states (epoch 0 never matches a launch), the control
   // block and the status words.
   if (cudaMemset(c->s.lb_states, 0, sizeof(unsigned long long) * c->states_words) != cudaSuccess ||

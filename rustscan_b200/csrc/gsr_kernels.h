@@ -170,7 +170,7 @@ cudaError_t inclusive_scan_u32_scratch(const uint32_t* in, uint32_t* out, uint32
 // offset, vcount[1..2]): what radix_sort_pairs on the depth keys and
 // launch_offsets give. For n Gaussians and a number of views that
 // order_fits_cluster accepts.
-bool cluster_sort_available();
+bool cluster_sort_available(int device);
 bool order_fits_cluster(uint32_t n, uint32_t views, const Scratch& s);
 cudaError_t launch_order_offsets(const ViewSet& vs, uint32_t n, FwdBufs& b, const Scratch& s, cudaStream_t st);
 // Per view: offset[r] = exclusive scan of count[perm[r]], sets vcount[1..2].

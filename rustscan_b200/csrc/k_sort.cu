@@ -7,11 +7,12 @@
 //  - one histogram pass over the keys computes the digit counts of every
 //    radix pass at once;
 //  - each radix pass is one persistent launch: blocks take 4096-key
-//    partitions by ticket, rank keys stably inside the block (peer lanes
-//    of a digit by match_any, or by one ballot per digit bit where the
-//    digits are near-random; warps in order), publish per-digit counts and look
-//    back across partitions for their global offsets, then scatter through
-//    shared memory so that every digit's run is written contiguously;
+//    partitions by ticket, rank keys stably inside the block (the peer lanes
+//    of a digit from a word per digit that they set their bit in; warps in
+//    order), publish per-digit counts and look back across partitions for
+//    their global offsets, then scatter through shared memory so that every
+//    digit's run is written contiguously. A block whose segment has no
+//    partition left takes those of the other segments;
 //  - scans are single-pass with the same look-back.
 // Keys are u32; `bits` (from bit shift0) set the passes: ceil(bits / 8)
 // passes of equal digits of at most 8 bits (12 bits: two 6-bit passes, whose
@@ -20,6 +21,7 @@
 // sorted alone (the binning packs tile id and compact index into one key
 // when both fit in 32 bits).
 #include <algorithm>
+#include <atomic>
 
 #include <cooperative_groups.h>
 
@@ -34,6 +36,7 @@ constexpr int kSortItems = 16;
 constexpr int kSortTile = kSortThreads * kSortItems;  // 4096
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kWarpKeys = kSortItems * 32;  // 512 keys per warp
+constexpr uint64_t kSortManyParts = 2048;
 
 __device__ __forceinline__ uint32_t seg_count(const uint32_t* counts, uint32_t stride, uint32_t seg, uint32_t n_host,
                                               uint64_t cap) {
@@ -92,9 +95,18 @@ struct SortPassArgs {
   DevStatus* status;
 };
 
-// KV: values travel with the keys; otherwise the keys are sorted alone.
-template <bool KV>
-__global__ void __launch_bounds__(kSortThreads, KV ? 2 : 4) sort_pass_kernel(SortPassArgs a) {
+// KV: values travel with the keys; otherwise the keys are sorted alone. What
+// bounds it is the latency of the ranking's rounds and, in the first
+// partitions, of the look-back. Ranking by a shared-memory word per digit
+// (about 12 ALU instructions a round, where a ballot per digit bit takes 40 and
+// match_any slows with the distinct digits) took the tile sort of 8 views of
+// 1M Gaussians from 0.986 to 0.754 ms and their depth sort from 0.302 to
+// 0.285; blocks that help other segments then took the tile sort to 0.628 and
+// the depth sort to 0.249, and the tile sort of 16 uneven views of 2M from 5.50
+// to 2.52 ms.
+// RES: blocks resident per SM (the register bound).
+template <bool KV, int RES>
+__global__ void __launch_bounds__(kSortThreads, RES) sort_pass_kernel(SortPassArgs a) {
   __shared__ uint32_t s_keys[kSortTile];
   __shared__ uint32_t s_vals[KV ? kSortTile : 1];
   __shared__ uint32_t s_whist[kSortWarps][256];
@@ -105,114 +117,116 @@ __global__ void __launch_bounds__(kSortThreads, KV ? 2 : 4) sort_pass_kernel(Sor
   __shared__ uint32_t s_dropped;
   const uint32_t epoch = epoch_begin(a.ctl);
   const unsigned long long tag = (unsigned long long)(epoch & 0x3fffffffu) << 34;
-  const int dbits = __popc(a.dmask);
-  const int rbits = dbits + (a.drop ? 1 : 0);  // digit bits ranked (the dropped keys' digit is dmask + 1)
   const uint32_t kDropDigit = a.dmask + 1u;
-  const uint32_t seg = blockIdx.y;
-  const uint32_t n = seg_count(a.counts, a.count_stride, seg, a.n_host, a.cap);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t lt_mask = (1u << lane) - 1u;
-  const uint32_t* kin = a.keys_in + (size_t)seg * a.seg_stride;
-  const uint32_t* vin = a.vals_in ? a.vals_in + (size_t)seg * a.seg_stride : nullptr;
-  uint32_t* kout = a.keys_out + (size_t)seg * a.seg_stride;
-  uint32_t* vout = a.vals_out + (size_t)seg * a.seg_stride;
-  unsigned long long* states = a.states + (size_t)seg * a.parts_cap * 256;
-  const uint32_t* gbase = a.base + (size_t)seg * 1024 + a.pass * 256;
-  for (;;) {
-    const uint32_t part = next_ticket(a.ctl, seg, &s_ticket);
-    if ((uint64_t)part * kSortTile >= n) break;
-    const uint32_t tile0 = part * kSortTile;
-    uint32_t key[kSortItems], val[kSortItems], lrank[kSortItems];
+  // A block starts on its own segment and helps the others when that one has
+  // no partition left: segments are of uneven length.
+  for (uint32_t turn = 0; turn < gridDim.y; ++turn) {
+    const uint32_t seg = blockIdx.y + turn < gridDim.y ? blockIdx.y + turn : blockIdx.y + turn - gridDim.y;
+    const uint32_t n = seg_count(a.counts, a.count_stride, seg, a.n_host, a.cap);
+    const uint32_t* kin = a.keys_in + (size_t)seg * a.seg_stride;
+    const uint32_t* vin = a.vals_in ? a.vals_in + (size_t)seg * a.seg_stride : nullptr;
+    uint32_t* kout = a.keys_out + (size_t)seg * a.seg_stride;
+    uint32_t* vout = a.vals_out + (size_t)seg * a.seg_stride;
+    unsigned long long* states = a.states + (size_t)seg * a.parts_cap * 256;
+    const uint32_t* gbase = a.base + (size_t)seg * 1024 + a.pass * 256;
+    for (;;) {
+      const uint32_t part = next_ticket(a.ctl, seg, &s_ticket);
+      if ((uint64_t)part * kSortTile >= n) break;
+      const uint32_t tile0 = part * kSortTile;
+      uint32_t key[kSortItems];
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
-      const uint32_t idx = tile0 + warp * kWarpKeys + i * 32 + lane;
-      const bool ok = idx < n;
-      key[i] = ok ? kin[idx] : 0xffffffffu;
-      val[i] = (KV && ok) ? (vin ? vin[idx] : idx) : 0u;
-    }
-    for (int j = lane; j < 256; j += 32) s_whist[warp][j] = 0;
-    __syncwarp();
-    // Stable rank within the warp: rounds in order, lanes in order.
+      for (int i = 0; i < kSortItems; ++i) {
+        const uint32_t idx = tile0 + warp * kWarpKeys + i * 32 + lane;
+        key[i] = idx < n ? kin[idx] : 0xffffffffu;
+      }
+      uint32_t* peer = s_keys + warp * 256;  // per digit, the lanes of a round that hold it
+      for (int j = lane; j < 256; j += 32) s_whist[warp][j] = peer[j] = 0;
+      __syncwarp();
+      // Stable rank within the warp: rounds in order, lanes in order.
+      uint32_t lrank[kSortItems / 2];  // two 16-bit ranks a word
 #pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
-      const uint32_t idx = tile0 + warp * kWarpKeys + i * 32 + lane;
-      const bool ok = idx < n;
-      uint32_t d, peers;
-      if (KV) {
-        // Near-random digits (depth keys): one ballot per digit bit.
-        d = (a.drop && key[i] == 0xffffffffu) ? kDropDigit : (key[i] >> a.shift) & a.dmask;
-        const uint32_t okm = __ballot_sync(0xffffffffu, ok);  // every lane, also past the end
-        peers = ok ? okm : (1u << lane);
-#pragma unroll
-        for (int bit = 0; bit < 8; ++bit) {
-          if (bit < rbits) {
-            const bool set = (d >> bit) & 1u;
-            const uint32_t bb = __ballot_sync(0xffffffffu, set);
-            peers &= set ? bb : ~bb;
-          }
+      for (int i = 0; i < kSortItems; ++i) {
+        const bool ok = tile0 + warp * kWarpKeys + i * 32 + lane < n;
+        const uint32_t d = (a.drop && key[i] == 0xffffffffu) ? kDropDigit : (key[i] >> a.shift) & a.dmask;
+        if (ok) atomicOr(peer + d, 1u << lane);
+        __syncwarp();
+        uint32_t peers = 0, b = 0;
+        if (ok) {
+          peers = peer[d];
+          b = s_whist[warp][d];
         }
-      } else {
-        // Clustered digits (tile ids of neighbouring boxes): few distinct
-        // values per warp, where match_any is cheaper.
-        d = ok ? ((a.drop && key[i] == 0xffffffffu) ? kDropDigit : ((key[i] >> a.shift) & a.dmask)) : (256u + lane);
-        peers = __match_any_sync(0xffffffffu, d);
+        const uint32_t below = peers & lt_mask;
+        __syncwarp();
+        if (ok && below == 0) {
+          s_whist[warp][d] = b + __popc(peers);
+          peer[d] = 0;
+        }
+        __syncwarp();
+        const uint32_t r = b + __popc(below);
+        if (i & 1)
+          lrank[i / 2] |= r << 16;
+        else
+          lrank[i / 2] = r;
       }
-      const uint32_t below = peers & lt_mask;
-      uint32_t b = 0;
-      if (ok) b = s_whist[warp][d];
-      __syncwarp();
-      if (ok && below == 0) s_whist[warp][d] = b + __popc(peers);
-      __syncwarp();
-      lrank[i] = b + __popc(below);
-    }
-    __syncthreads();
-    // Per digit (one per thread): warp offsets and the block count.
-    const uint32_t d = threadIdx.x;
-    uint32_t sum = 0;
+      uint32_t val[KV ? kSortItems : 1];  // loaded late: the ranking needs the registers
+      if (KV) {
 #pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) {
-      const uint32_t t = s_whist[w][d];
-      s_whist[w][d] = sum;
-      sum += t;
-    }
-    // The digit counts are published before the block scan, so that later
-    // partitions can sum past this one as early as possible; only the
-    // pass's digits look back.
-    if (d <= a.dmask) st_volatile64(states + (size_t)part * 256 + d, tag | (part == 0 ? kFlagPre : kFlagAgg) | sum);
-    uint32_t tot;
-    const uint32_t dstart = block_exclusive_scan(sum, s_scan, &tot);
-    const uint32_t excl = d <= a.dmask ? lookback(states + d, 256, part, sum, epoch, a.status, kWaitSort) : 0u;
-    s_dstart[d] = dstart;
-    s_gbase[d] = gbase[d] + excl - dstart;
-    // The dropped keys are placed last in the block and never written (one
-    // thread sets the count: the drop digit's, or thread 0 when nothing drops).
-    if (d == (a.drop ? kDropDigit : 0u)) s_dropped = a.drop ? sum : 0u;
-    // This partition writes digit d's keys to gbase[d] + excl onwards; a
-    // position past the segment would mean the digit histogram did not
-    // describe these keys. Such a partition writes nothing and is reported
-    // through the status words.
-    const bool outside = d <= a.dmask && sum != 0u && s_gbase[d] + dstart + sum > n;  // each term is below 2^30
-    if (__syncthreads_or(outside)) {
-      if (threadIdx.x == 0) atomicOr(&a.status->internal, 1u);
-      continue;
-    }
-#pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
-      const uint32_t idx = tile0 + warp * kWarpKeys + i * 32 + lane;
-      if (idx < n) {
-        const uint32_t dd = (a.drop && key[i] == 0xffffffffu) ? kDropDigit : (key[i] >> a.shift) & a.dmask;
-        const uint32_t pos = s_dstart[dd] + s_whist[warp][dd] + lrank[i];
-        s_keys[pos] = key[i];
-        if (KV) s_vals[pos] = val[i];
+        for (int i = 0; i < kSortItems; ++i) {
+          const uint32_t idx = tile0 + warp * kWarpKeys + i * 32 + lane;
+          val[i] = idx < n ? (vin ? vin[idx] : idx) : 0u;
+        }
       }
-    }
-    __syncthreads();
-    const uint32_t nvalid = min((uint32_t)kSortTile, n - tile0) - s_dropped;
-    for (uint32_t j = threadIdx.x; j < nvalid; j += kSortThreads) {
-      const uint32_t k = s_keys[j];
-      const uint32_t dst = s_gbase[(k >> a.shift) & a.dmask] + j;
-      kout[dst] = k;
-      if (KV) vout[dst] = s_vals[j];
+      __syncthreads();
+      // Per digit (one per thread): warp offsets and the block count.
+      const uint32_t d = threadIdx.x;
+      uint32_t sum = 0;
+#pragma unroll
+      for (int w = 0; w < kSortWarps; ++w) {
+        const uint32_t t = s_whist[w][d];
+        s_whist[w][d] = sum;
+        sum += t;
+      }
+      // The digit counts are published before the block scan, so that later
+      // partitions can sum past this one as early as possible; only the
+      // pass's digits look back.
+      if (d <= a.dmask) st_volatile64(states + (size_t)part * 256 + d, tag | (part == 0 ? kFlagPre : kFlagAgg) | sum);
+      uint32_t tot;
+      const uint32_t dstart = block_exclusive_scan(sum, s_scan, &tot);
+      const uint32_t excl = d <= a.dmask ? lookback(states + d, 256, part, sum, epoch, a.status, kWaitSort) : 0u;
+      s_dstart[d] = dstart;
+      s_gbase[d] = gbase[d] + excl - dstart;
+      // The dropped keys are placed last in the block and never written (one
+      // thread sets the count: the drop digit's, or thread 0 when nothing drops).
+      if (d == (a.drop ? kDropDigit : 0u)) s_dropped = a.drop ? sum : 0u;
+      // This partition writes digit d's keys to gbase[d] + excl onwards; a
+      // position past the segment would mean the digit histogram did not
+      // describe these keys. Such a partition writes nothing and is reported
+      // through the status words.
+      const bool outside = d <= a.dmask && sum != 0u && s_gbase[d] + dstart + sum > n;  // each term is below 2^30
+      if (__syncthreads_or(outside)) {
+        if (threadIdx.x == 0) atomicOr(&a.status->internal, 1u);
+        continue;
+      }
+#pragma unroll
+      for (int i = 0; i < kSortItems; ++i) {
+        const uint32_t idx = tile0 + warp * kWarpKeys + i * 32 + lane;
+        if (idx < n) {
+          const uint32_t dd = (a.drop && key[i] == 0xffffffffu) ? kDropDigit : (key[i] >> a.shift) & a.dmask;
+          const uint32_t pos = s_dstart[dd] + s_whist[warp][dd] + ((lrank[i / 2] >> (16 * (i & 1))) & 0xffffu);
+          s_keys[pos] = key[i];
+          if (KV) s_vals[pos] = val[KV ? i : 0];
+        }
+      }
+      __syncthreads();
+      const uint32_t nvalid = min((uint32_t)kSortTile, n - tile0) - s_dropped;
+      for (uint32_t j = threadIdx.x; j < nvalid; j += kSortThreads) {
+        const uint32_t k = s_keys[j];
+        const uint32_t dst = s_gbase[(k >> a.shift) & a.dmask] + j;
+        kout[dst] = k;
+        if (KV) vout[dst] = s_vals[j];
+      }
     }
   }
   epoch_end(a.ctl, epoch);
@@ -315,18 +329,20 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(ScanArgs a) {
 // stably (as sort_pass_kernel does), the CTAs send their digit counts to one
 // another, and every pair is stored straight to its place in the CTA that
 // owns it. Two cluster barriers per pass take the place of a launch and a
-// look-back. What bounds it, in cycles of one SM: about 1500 per round of 1024
-// pairs to rank, 1300 to send them (single 8-byte stores), 2000 per barrier.
+// look-back. What bounds it is latency: about 2000 cycles per barrier, and per
+// 1024 pairs of a CTA 1300 to send them (single 8-byte stores) besides the
+// ranking.
 // ---------------------------------------------------------------------------
 constexpr int kClusterThreads = 1024;
 constexpr int kClusterWarps = kClusterThreads / 32;
 constexpr int kClusterDigits = 512;  // of at most 9 bits
 // Up to 13 pairs per thread of 16 CTAs, and for more than 4 views (the GPU
 // holds about so many of these clusters at a time) few enough pairs that the
-// later waves stay cheap. Depth order and offsets by the radix passes and by
-// the cluster, in us: one view of 14k visible Gaussians 85 and 34, of 55k 93
-// and 44, of 149k 102 and 81, of 179k 106 and 103; 8 views of 55k 106 and 77,
-// of 97k 116 and 107, of 149k 143 and 153; 16 views of 55k 118 and 119.
+// later waves stay cheap. Depth order and offsets by the radix passes (as they
+// were when this line was drawn) and by the cluster, in us: one view of 14k
+// visible Gaussians 85 and 34, of 55k 93 and 42, of 149k 102 and 75, of 179k
+// 97 and 98; 8 views of 55k 106 and 71, of 97k 116 and 97, of 149k 143 and
+// 153; 16 views of 55k 118 and 119.
 constexpr uint32_t kClusterMaxKeys = 16u * kClusterThreads * 13u;
 constexpr uint64_t kClusterMaxWaveKeys = 300000;
 
@@ -342,7 +358,10 @@ struct ClusterSortArgs {
 };
 
 template <int C, int IT> struct ClusterSortSmem {
-  uint2 pair[IT * kClusterThreads];
+  union {
+    uint2 pair[IT * kClusterThreads];
+    uint32_t peer[kClusterWarps][kClusterDigits];  // ranking, when the pairs are in registers
+  };
   uint16_t whist[kClusterWarps][kClusterDigits];  // per warp: digit counts, then starts
   uint32_t counts[C][kClusterDigits];             // every CTA's digit counts of the pass
   uint32_t base[kClusterDigits];
@@ -408,7 +427,11 @@ __global__ void __launch_bounds__(kClusterThreads, 1) cluster_sort_kernel(Cluste
 #pragma unroll
   for (int i = 0; i < IT; ++i) kv[i].x -= lo;
   for (uint32_t shift = 0; shift < bits; shift += dbits) {
-    for (uint32_t d = lane; d < digits; d += 32u) S.whist[warp][d] = 0;
+    uint32_t* peer = S.peer[warp];  // per digit, the lanes of a round that hold it
+    for (uint32_t d = lane; d < digits; d += 32u) {
+      S.whist[warp][d] = 0;
+      peer[d] = 0;
+    }
     __syncwarp();
     // Stable rank within the warp: rounds in order, lanes in order.
     uint32_t ranks[(IT + 1) / 2];  // two 16-bit ranks a word
@@ -417,18 +440,20 @@ __global__ void __launch_bounds__(kClusterThreads, 1) cluster_sort_kernel(Cluste
       uint32_t r = 0;
       if ((uint32_t)i < it) {
         const bool ok = at0 + 32u * i < mine;
-        const uint32_t d = ok ? (kv[i].x >> shift) & dmask : 0u;
-        uint32_t peers = __ballot_sync(0xffffffffu, ok);
-#pragma unroll
-        for (int bit = 0; bit < 9; ++bit) {
-          const bool set = (d >> bit) & 1u;
-          const uint32_t bb = __ballot_sync(0xffffffffu, set);
-          peers &= set ? bb : ~bb;
+        const uint32_t d = (kv[i].x >> shift) & dmask;
+        if (ok) atomicOr(peer + d, 1u << lane);
+        __syncwarp();
+        uint32_t peers = 0, b = 0;
+        if (ok) {
+          peers = peer[d];
+          b = S.whist[warp][d];
         }
         const uint32_t below = peers & ((1u << lane) - 1u);
-        const uint32_t b = ok ? S.whist[warp][d] : 0u;
         __syncwarp();
-        if (ok && below == 0) S.whist[warp][d] = (uint16_t)(b + __popc(peers));
+        if (ok && below == 0) {
+          S.whist[warp][d] = (uint16_t)(b + __popc(peers));
+          peer[d] = 0;
+        }
         __syncwarp();
         r = b + __popc(below);
       }
@@ -479,6 +504,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) cluster_sort_kernel(Cluste
       const uint32_t j = at0 + 32u * i;
       if ((uint32_t)i < it && j < mine) kv[i] = S.pair[j];
     }
+    __syncthreads();  // the next pass ranks in the pairs' memory
   }
   // Depth order out, and the exclusive scan of the counts along it: a warp's
   // pairs are consecutive, rounds in order.
@@ -630,11 +656,19 @@ cudaError_t radix_sort_pairs(const uint32_t* keys_in, const uint32_t* vals_in, u
     a.parts_cap = parts_cap;
     a.ctl = s.ctl;
     a.status = s.status;
-    dim3 grid(persistent_blocks(s.num_sms, segments, kv ? 3 : 4), segments);
-    if (kv)
-      sort_pass_kernel<true><<<grid, kSortThreads, 0, st>>>(a);
+    // Three blocks of the pair kernel per SM spill a little; it pays once there
+    // are partitions enough to fill them several times (16 uneven views of 2M
+    // Gaussians: tile sort 2.78 -> 2.52 ms, depth sort 0.93 -> 0.90) and costs
+    // where few partitions wait for one another (one view of 345k keys 82 -> 97
+    // us). The keys-only kernel runs 4.
+    const int res = !kv ? 4 : (uint64_t)parts_cap * segments > kSortManyParts ? 3 : 2;
+    dim3 grid(persistent_blocks(s.num_sms, segments, res), segments);
+    if (res == 4)
+      sort_pass_kernel<false, 4><<<grid, kSortThreads, 0, st>>>(a);
+    else if (res == 3)
+      sort_pass_kernel<true, 3><<<grid, kSortThreads, 0, st>>>(a);
     else
-      sort_pass_kernel<false><<<grid, kSortThreads, 0, st>>>(a);
+      sort_pass_kernel<true, 2><<<grid, kSortThreads, 0, st>>>(a);
     ki = ko;
     vi = vo;
   }
@@ -686,11 +720,17 @@ cudaError_t inclusive_scan_u32_scratch(const uint32_t* in, uint32_t* out, uint32
   return cudaGetLastError();
 }
 
-bool cluster_sort_available() {
+bool cluster_sort_available(int device) {
+  // A property of the device (0: not asked yet, 1: yes, 2: no), asked once per
+  // process: the occupancy query can take milliseconds.
+  static std::atomic<int> known[64];
+  const bool listed = device >= 0 && device < 64;
+  if (listed && known[device].load() != 0) return known[device].load() == 1;
   bool ok = true;
   for (uint32_t it : {2u, 5u, 8u, 13u})
     ok = ok && cluster_sort_pick(it * 16u * kClusterThreads, ClusterSortArgs{}, 1, nullptr, true) == cudaSuccess;
   (void)cudaGetLastError();
+  if (listed) known[device].store(ok ? 1 : 2);
   return ok;
 }
 
