@@ -159,8 +159,9 @@ gsr_status allocate(gsr_ctx* c) {
             dalloc(c, &b.ranges, nv * 2 * T) && dalloc(c, &b.tfinal, nv * P) && dalloc(c, &b.last, nv * P) &&
             dalloc(c, &b.ncontrib, nv * P) && dalloc(c, &b.nvisit, nv * P) && dalloc(c, &b.visible_c, nv * V) &&
             dalloc(c, &b.sgrad, nv * V * 3) && dalloc(c, &b.pair, nv * V * 6) && dalloc(c, &b.vcount, nv * 4) &&
-            dalloc(c, &b.tile_hist, nv * T) && dalloc(c, &b.hitw, nv * I) && dalloc(c, &b.sched_order, nv * T) &&
-            dalloc(c, &b.sched_lcount, 32) && dalloc(c, &b.sched_ticket, 1);
+            dalloc(c, &b.tile_hist, nv * T) && dalloc(c, &b.hitw, nv * I + 4) && dalloc(c, &b.sched_order, nv * T) &&
+            dalloc(c, &b.sched_lcount, 32 + 2 * kFwdSplitTiles) && dalloc(c, &b.sched_ticket, 1);
+  b.tile_sync = b.sched_lcount + 32;
   // Backward work items: the tiles, or the segments of a launch of few tiles.
   b.sched_items_cap = std::max<uint64_t>(nv * T, kSegItems);
   ok = ok && dalloc(c, &b.sched_lists, 32 * b.sched_items_cap);
@@ -256,6 +257,7 @@ gsr_status build_views(gsr_ctx* c, const gsr_camera* cams, uint32_t n_views, std
   vs.batch = c->cfg.batch;
   vs.total_tiles = tile_base;
   vs.max_tiles = max_tiles;
+  vs.n_splats = 0;
   // The default runs the backward persistently and the forward as a grid:
   // on the 8-view 1280x720 step the cost order shortens the backward by 5%,
   // while the forward, whose cost (entries up to saturation) the list length
@@ -304,6 +306,7 @@ gsr_status forward_impl(gsr_ctx* c, const gsr_splats* sp, const gsr_camera* cams
   ViewSet vs;
   rs = build_views(c, cams, n_views, desc, vs);
   if (rs != GSR_OK) return rs;
+  vs.n_splats = sp->n;
   GSR_CUDA(c, launch_set_views(c->d_views, desc.data(), n_views, st));
   const SplatsDev sd = splats_dev(c, sp);
   FwdBufs& b = c->b;

@@ -47,6 +47,7 @@ struct FwdBufs {
   uint32_t* sched_order;   // [views * Tcap] persistent forward: work items in issue order
   uint32_t* sched_lists;   // [32][sched_items_cap] work items by the bit length of their backward cost
   uint32_t* sched_lcount;  // [32] items in each of those lists (appended by the forward)
+  uint32_t* tile_sync;     // [kFwdSplitTiles][2] split forward, after sched_lcount: largest last contributor, CTAs done
   uint32_t* sched_ticket;  // [1] next ticket a persistent raster CTA takes
   uint64_t sched_items_cap;
   float4* ckpt;            // [kSegItems][256] per (tile, segment) and pixel: transmittance after it, colour behind it
@@ -72,11 +73,20 @@ struct ViewSet {
   uint32_t batch;         // Gaussians per shared-memory batch of the rasterizer (0: tuned defaults)
   uint32_t total_tiles;   // sum over views of tiles_x * tiles_y
   uint32_t max_tiles;     // max over views
+  uint32_t n_splats;      // Gaussians of the launch
   int persistent;         // kPersist* bits: raster kernels whose CTAs take cost-ordered items persistently
 };
 // (Tile, segment) items of a segmented 16x16 backward: a launch of few tiles
 // cuts every tile's list into up to kSegMax segments, kSegItems over all tiles.
 constexpr uint32_t kSegItems = 16384, kSegMax = 64;
+// A launch of at most so many 16x16 tiles, with at least so many Gaussians per
+// tile, blends each 8x8 block of a tile in a CTA of its own: the longest tiles'
+// work then spreads over four SMs and is cut into finer lists. It costs a
+// launch (clearing the hit bits) and stages each entry four times. Blending
+// without and with, in us: 300 tiles over 74k Gaussians 116 and 83, 400 over
+// 50k 101 and 78, 900 over 120k 100 and 92, 1024 over 200k 117 and 108, 1200
+// over 200k 100 and 100, 2025 over 300k 124 and 132; 1024 over 10k 33 and 37.
+constexpr uint32_t kFwdSplitTiles = 1024, kFwdSplitSplats = 32;
 
 // Bits of ViewSet::persistent (otherwise one CTA per work item).
 constexpr int kPersistFwd = 1, kPersistBwd = 2;

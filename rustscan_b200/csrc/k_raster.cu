@@ -73,6 +73,7 @@ struct RasterArgs {
   const float* v_rgba;
   int ref_mode;
   int det;
+  int split;    // forward: a CTA per 8x8 block of a 16x16 tile
   int persist;  // 0: one CTA per item; 1: persistent, items from sched_order; 2: persistent, items from the cost lists
 };
 
@@ -125,9 +126,12 @@ __device__ __forceinline__ uint32_t take_item(const RasterArgs& a, uint32_t roun
   __syncthreads();
   return *s_item;
 }
+// PARTS: items per tile, in its place of the order.
+template <int PARTS>
 __device__ __forceinline__ uint32_t next_item(const RasterArgs& a, uint32_t round, uint32_t* s_item) {
   return take_item(a, round, s_item, [&](uint32_t slot) {
-    return slot < a.vs.total_tiles ? a.b.sched_order[slot] : kNoItem;
+    const uint32_t at = slot / PARTS;
+    return at < a.vs.total_tiles ? a.b.sched_order[at] * PARTS + slot % PARTS : kNoItem;
   });
 }
 // FIRST (launches whose items fit the resident CTAs a few times over): a CTA's
@@ -205,9 +209,9 @@ template <int TW, int PPL> struct WarpBlock {
   __device__ static int y0(int w) { return (w / kWarpsX) * kRows; }
 };
 
-// The 8x8 warp blocks of a tile at (tx0, ty0) that a Gaussian can reach: bit
-// w set unless sigma exceeds the cut over the whole rectangle of block w's
-// pixel centres. The smallest value of a positive-definite quadratic over a
+// The warp blocks (8 columns, ROWS rows) of a tile at (tx0, ty0) that a
+// Gaussian can reach: bit w set unless sigma exceeds the cut over the whole
+// rectangle of block w's pixel centres. The smallest value of a positive-definite quadratic over a
 // rectangle that does not hold its centre lies on an edge facing the centre,
 // so two clamped edge minima give it. The test errs on the side of keeping:
 // sigma as the pixels evaluate it (and this minimum) is within 10 units of
@@ -215,7 +219,7 @@ template <int TW, int PPL> struct WarpBlock {
 // cut itself lies kRejectMargin above any sigma that can contribute. A conic
 // that float arithmetic cannot tell from an indefinite one, or a value that is
 // not a number, keeps every block.
-template <int TW, int NW>
+template <int TW, int NW, int ROWS>
 __device__ __forceinline__ uint32_t reached_blocks(float x, float y, float a, float b, float c, float cut, float tx0,
                                                    float ty0) {
   uint32_t mask = (1u << NW) - 1u;
@@ -224,8 +228,9 @@ __device__ __forceinline__ uint32_t reached_blocks(float x, float y, float a, fl
 #pragma unroll
   for (int w = 0; w < NW; ++w) {
     // Offsets mean - centre over the block's columns and rows.
-    const float x1 = x - (tx0 + (float)(8 * (w % (TW / 8))) + 0.5f), x0 = x1 - 7.f;
-    const float y1 = y - (ty0 + (float)(8 * (w / (TW / 8))) + 0.5f), y0 = y1 - 7.f;
+    constexpr int S = 8 / ROWS;  // warps per 8x8 block
+    const float x1 = x - (tx0 + (float)(8 * (w / S % (TW / 8))) + 0.5f), x0 = x1 - 7.f;
+    const float y1 = y - (ty0 + (float)(8 * (w / S / (TW / 8)) + ROWS * (w % S)) + 0.5f), y0 = y1 - (float)(ROWS - 1);
     const float nx = fminf(fmaxf(0.f, x0), x1), ny = fminf(fmaxf(0.f, y0), y1);
     const float ey = fminf(fmaxf(kc * nx, y0), y1), ex = fminf(fmaxf(ka * ny, x0), x1);
     const float q1 = fmaf(fmaf(a, nx, b2 * ey), nx, c * ey * ey);
@@ -272,6 +277,11 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+// The same operations for a lane with one pixel.
+__device__ __forceinline__ float add2(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float mul2(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float fma2(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float neg2(float a) { return -a; }
 
 // blend_sigma_shared for the two pixels of a pair (same column: same t1,
 // t2): the same operations in the same order, each half rounded on its own.
@@ -306,6 +316,38 @@ __device__ __forceinline__ float2 blend_exp2(float2 sigma) {
   p = fma2(p, r, f2(1.0f));
   return make_float2(__uint_as_float(__float_as_uint(p.x) + ex), __uint_as_float(__float_as_uint(p.y) + ey));
 }
+__device__ __forceinline__ float blend_exp2(float sigma) {
+  const float x = -sigma;
+  const float t = __fmaf_rn(x, bexp::kLog2e, bexp::kMagic);
+  const float n = __fadd_rn(t, -bexp::kMagic);
+  float r = __fmaf_rn(-n, bexp::kLn2Hi, x);
+  r = __fmaf_rn(-n, bexp::kLn2Lo, r);
+  float p = bexp::kC6;
+  p = __fmaf_rn(p, r, bexp::kC5);
+  p = __fmaf_rn(p, r, bexp::kC4);
+  p = __fmaf_rn(p, r, bexp::kC3);
+  p = __fmaf_rn(p, r, bexp::kC2);
+  p = __fmaf_rn(p, r, 1.0f);
+  p = __fmaf_rn(p, r, 1.0f);
+  return __uint_as_float(__float_as_uint(p) + (__float_as_uint(t) << 23));
+}
+
+// The pixels of a forward lane: a pair in one register pair, or one.
+template <int PX> struct Lane;
+template <> struct Lane<2> {
+  using V = float2;
+  __device__ static V all(float x) { return make_float2(x, x); }
+  __device__ static V of(float2 twice) { return twice; }
+  __device__ static V make(const float (&x)[2]) { return make_float2(x[0], x[1]); }
+  __device__ static float get(V v, int h) { return h ? v.y : v.x; }
+};
+template <> struct Lane<1> {
+  using V = float;
+  __device__ static V all(float x) { return x; }
+  __device__ static V of(float2 twice) { return twice.x; }
+  __device__ static V make(const float (&x)[1]) { return x[0]; }
+  __device__ static float get(V v, int) { return v; }
+};
 
 // Entries per segment of a list of `len` entries cut into at most k segments:
 // 32 where that covers the list, else 64 (the last segment takes the rest).
@@ -355,12 +397,22 @@ constexpr int kFwdThreadsPerSm = 768;
 // running totals, so that what lies far behind keeps its relative accuracy.
 // The next batch's records are then also loaded while the current one is
 // walked, since few warps are there to hide the loads.
-template <int TW, int TH, int BATCH, bool CKPT>
-__global__ void __launch_bounds__(TW* TH / 2, CKPT ? 4 : kFwdThreadsPerSm / (TW * TH / 2)) raster_fwd_kernel(RasterArgs a) {
-  constexpr int NT = TW * TH / 2;
+// SPLIT (16x16 tiles, with CKPT): a CTA per 8x8 block of a tile, two warps with
+// one pixel per lane, each walking the entries that reach its 8x4 strip (see
+// kFwdSplitTiles). The four CTAs of a tile set their hit bits one by one, and
+// the last of them lists the tile for the backward.
+template <int TW, int TH, int BATCH, bool CKPT, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 64 : TW * TH / 2, SPLIT ? 8 : CKPT ? 4 : kFwdThreadsPerSm / (TW * TH / 2))
+    raster_fwd_kernel(RasterArgs a) {
+  constexpr int PX = SPLIT ? 1 : 2;  // pixels per lane
+  using L = Lane<PX>;
+  using V = typename L::V;
+  constexpr int NT = SPLIT ? 64 : TW * TH / 2;
   constexpr int NW = NT / 32;
+  constexpr int S = 2 / PX;                   // warps per 8x8 block
+  constexpr int BW = SPLIT ? 8 : TW;          // width of the CTA's pixel area
   constexpr int kSI = (BATCH + NT - 1) / NT;  // entries a thread stages per batch
-  static_assert(NW <= 4 && TW % 8 == 0 && TH % 8 == 0, "hit bits of at most four 8x8 blocks");
+  static_assert(NW / S <= 4 && TW % 8 == 0 && TH % 8 == 0, "hit bits of at most four 8x8 blocks");
   __shared__ FwdEntry s_e[BATCH + 1];  // the last one is never taken: it pads the lists
   __shared__ uint8_t s_mask[BATCH];
   __shared__ __align__(8) uint16_t s_list[NW][BATCH + kFwdUnroll];  // byte offsets into s_e
@@ -371,18 +423,29 @@ __global__ void __launch_bounds__(TW* TH / 2, CKPT ? 4 : kFwdThreadsPerSm / (TW 
     s_e[BATCH] = FwdEntry{};  // sigma 0, opacity 0: alpha 0
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int half = warp % S;  // SPLIT: the block's rows y + 4 half
   uint16_t* list = s_list[warp];
   for (uint32_t round = 0;; ++round) {
-    const uint32_t item = next_item(a, round, &s_item);
-    if (item == kNoItem) break;
+    const uint32_t work = next_item<SPLIT ? 4 : 1>(a, round, &s_item);
+    if (work == kNoItem) break;
+    const uint32_t item = SPLIT ? work / 4 : work;
+    const int block = SPLIT ? (int)(work % 4) : warp;  // 8x8 block of the tile
     const uint32_t v = find_view(a.vs, item);
     const ViewDesc& vd = a.vs.views[v];
     const uint32_t t = item - vd.tile_base;
     const uint32_t tx = t % vd.tiles_x, ty = t / vd.tiles_x;
-    const uint32_t px = tx * TW + WarpBlock<TW, 2>::x0(warp) + (lane & 7);
-    const uint32_t py = ty * TH + WarpBlock<TW, 2>::y0(warp) + (lane >> 3);
+    const uint32_t px = tx * TW + WarpBlock<TW, 2>::x0(block) + (lane & 7);
+    const uint32_t py = ty * TH + WarpBlock<TW, 2>::y0(block) + (lane >> 3) + 4 * half;
     const float pcx = (float)px + 0.5f;
-    const float2 npcy = make_float2(-((float)py + 0.5f), -((float)(py + 4) + 0.5f));
+    float rows[PX], first[PX];
+    bool inside[PX];
+#pragma unroll
+    for (int h = 0; h < PX; ++h) {
+      rows[h] = -((float)(py + 4 * h) + 0.5f);
+      inside[h] = px < vd.w && py + 4 * h < vd.h;
+      first[h] = inside[h] ? 1.f : 0.f;  // a pixel outside the image starts saturated
+    }
+    const V npcy = L::make(rows);
     const uint32_t* ranges = slice(a.b.ranges, 2 * a.b.Tcap, v);
     const uint32_t s0 = ranges[2 * t], s1 = ranges[2 * t + 1];
     const uint32_t* vals = isect_index_src(a.b, v);
@@ -390,16 +453,22 @@ __global__ void __launch_bounds__(TW* TH / 2, CKPT ? 4 : kFwdThreadsPerSm / (TW 
     const float4* rec = slice(a.b.rec, a.b.Vcap * 3, v);
     uint8_t* vis = slice(a.b.visible_c, a.b.Vcap, v);
     uint8_t* hitw = slice(a.b.hitw, a.b.Icap, v);
-    const float tx0 = (float)(tx * TW), ty0 = (float)(ty * TH);
-    const bool in0 = px < vd.w && py < vd.h, in1 = px < vd.w && py + 4 < vd.h;
-    // A pixel outside the image starts saturated.
-    float2 T = make_float2(in0 ? 1.f : 0.f, in1 ? 1.f : 0.f);
-    float2 C0 = f2(0.f), C1 = f2(0.f), C2 = f2(0.f);
-    uint32_t last0 = 0, last1 = 0, nc0 = 0, nc1 = 0;
-    // Checkpoints of this tile, segment by segment: half h of thread t's pair
-    // at ck[segment * pixels + h * threads + t].
-    float4* ck = CKPT ? a.b.ckpt + (size_t)item * a.b.seg_k * (TW * TH) + threadIdx.x : nullptr;
-    float2 S0 = f2(0.f), S1 = f2(0.f), S2 = f2(0.f);  // colour added since the last checkpoint
+    // Corner of the CTA's pixel area.
+    const float tx0 = (float)(tx * TW + (SPLIT ? WarpBlock<TW, 2>::x0(block) : 0));
+    const float ty0 = (float)(ty * TH + (SPLIT ? WarpBlock<TW, 2>::y0(block) : 0));
+    V T = L::make(first), C0 = L::all(0.f), C1 = C0, C2 = C0;
+    uint32_t last[PX] = {}, nc[PX] = {};
+    auto saturated = [&] {
+      bool all = true;
+#pragma unroll
+      for (int h = 0; h < PX; ++h) all = all && L::get(T, h) < 1e-4f;
+      return all;
+    };
+    // Checkpoints of this tile, segment by segment: half h of lane l's pair in
+    // block q at ck[segment * pixels + h * pixels / 2 + 32 q + l].
+    constexpr int kHalf = TW * TH / 2;
+    float4* ck = CKPT ? a.b.ckpt + (size_t)item * a.b.seg_k * (TW * TH) + half * kHalf + block * 32 + lane : nullptr;
+    V S0 = C0, S1 = C0, S2 = C0;  // colour added since the last checkpoint
     uint32_t stored = 0;                              // checkpoints written
     const uint32_t seg_len = segment_len(s1 - s0, a.b.seg_k);
     struct Raw {
@@ -430,7 +499,7 @@ __global__ void __launch_bounds__(TW* TH / 2, CKPT ? 4 : kFwdThreadsPerSm / (TW 
       E.last = i + 1;
       *reinterpret_cast<uint32_t*>(E.hit) = 0u;
       E.cidx = r.c;
-      s_mask[j] = (uint8_t)reached_blocks<TW, NW>(r.r0.x, r.r0.y, r.r0.z, r.r0.w, r.r1.x, cut, tx0, ty0);
+      s_mask[j] = (uint8_t)reached_blocks<BW, NW, 8 / S>(r.r0.x, r.r0.y, r.r0.z, r.r0.w, r.r1.x, cut, tx0, ty0);
     };
     Raw next[CKPT ? kSI : 1];  // CKPT: this thread's entries of the next batch
     auto fetch = [&](uint32_t b0) {
@@ -461,58 +530,69 @@ __global__ void __launch_bounds__(TW* TH / 2, CKPT ? 4 : kFwdThreadsPerSm / (TW 
         for (uint32_t e = 0; e < cnt; e += kFwdUnroll) {
           const uint2 off2 = *reinterpret_cast<const uint2*>(list + e);
           const uint32_t off[kFwdUnroll] = {off2.x & 0xffffu, off2.x >> 16, off2.y & 0xffffu, off2.y >> 16};
-          float2 al[kFwdUnroll];
-          bool k0[kFwdUnroll], k1[kFwdUnroll];
+          V al[kFwdUnroll];
+          bool take[kFwdUnroll][PX];
 #pragma unroll
           for (int u = 0; u < kFwdUnroll; ++u) {
             const FwdEntry& E = *reinterpret_cast<const FwdEntry*>(reinterpret_cast<const char*>(s_e) + off[u]);
             const float dx = esub(E.x, pcx);
             const float t1 = emul(emul(E.a, dx), dx);
             const float t2 = emul(E.b2, dx);
-            const float2 dy = add2(E.y, npcy);
-            const float2 in = make_float2(fmaf(t2, dy.x, t1), fmaf(t2, dy.y, t1));
-            const float2 sg = mul2(f2(0.5f), fma2(mul2(E.c, dy), dy, in));  // sigma, as blend_sigma_shared
-            const float2 og = mul2(E.opac, blend_exp2(sg));
-            al[u] = make_float2(fminf(0.999f, og.x), fminf(0.999f, og.y));
+            const V dy = add2(L::of(E.y), npcy);
+            float in[PX], cl[PX];
+#pragma unroll
+            for (int h = 0; h < PX; ++h) in[h] = fmaf(t2, L::get(dy, h), t1);
+            // Sigma, as blend_sigma_shared.
+            const V sg = mul2(L::all(0.5f), fma2(mul2(L::of(E.c), dy), dy, L::make(in)));
+            const V og = mul2(L::of(E.opac), blend_exp2(sg));
             // 0 <= sigma <= cut in one unsigned comparison of the bits (sigma is
             // never -0; a negative one has the sign bit set) and alpha >= 1/255,
             // as blend_alpha_of decides.
             const uint32_t cut = __float_as_uint(E.cut);
-            k0[u] = __float_as_uint(sg.x) <= cut && al[u].x >= (float)(1.0 / 255.0);
-            k1[u] = __float_as_uint(sg.y) <= cut && al[u].y >= (float)(1.0 / 255.0);
+#pragma unroll
+            for (int h = 0; h < PX; ++h) {
+              cl[h] = fminf(0.999f, L::get(og, h));
+              take[u][h] = __float_as_uint(L::get(sg, h)) <= cut && cl[h] >= (float)(1.0 / 255.0);
+            }
+            al[u] = L::make(cl);
           }
 #pragma unroll
           for (int u = 0; u < kFwdUnroll; ++u) {
             FwdEntry& E = *reinterpret_cast<FwdEntry*>(reinterpret_cast<char*>(s_e) + off[u]);
-            const bool c0 = k0[u] && !(T.x < 1e-4f), c1 = k1[u] && !(T.y < 1e-4f);
-            const float2 am = make_float2(c0 ? al[u].x : 0.f, c1 ? al[u].y : 0.f);
-            const float2 w = mul2(am, T);
-            C0 = fma2(E.r, w, C0);  // blend_accum; the colours were clamped at staging
-            C1 = fma2(E.g, w, C1);
-            C2 = fma2(E.b, w, C2);
+            float am[PX];
+            bool any = false;
+#pragma unroll
+            for (int h = 0; h < PX; ++h) {
+              take[u][h] = take[u][h] && !(L::get(T, h) < 1e-4f);
+              am[h] = take[u][h] ? L::get(al[u], h) : 0.f;
+              any = any || take[u][h];
+            }
+            const V alpha = L::make(am);
+            const V w = mul2(alpha, T);
+            C0 = fma2(L::of(E.r), w, C0);  // blend_accum; the colours were clamped at staging
+            C1 = fma2(L::of(E.g), w, C1);
+            C2 = fma2(L::of(E.b), w, C2);
             if constexpr (CKPT) {
-              S0 = fma2(E.r, w, S0);
-              S1 = fma2(E.g, w, S1);
-              S2 = fma2(E.b, w, S2);
+              S0 = fma2(L::of(E.r), w, S0);
+              S1 = fma2(L::of(E.g), w, S1);
+              S2 = fma2(L::of(E.b), w, S2);
             }
-            T = mul2(T, add2(f2(1.f), neg2(am)));
-            if (c0 || c1) E.hit[warp] = 1;
-            if (c0) {
-              last0 = E.last;
-              ++nc0;
-            }
-            if (c1) {
-              last1 = E.last;
-              ++nc1;
-            }
+            T = mul2(T, add2(L::all(1.f), neg2(alpha)));
+            if (any) E.hit[SPLIT ? 0 : warp] = 1;
+#pragma unroll
+            for (int h = 0; h < PX; ++h)
+              if (take[u][h]) {
+                last[h] = E.last;
+                ++nc[h];
+              }
           }
-          if (__all_sync(0xffffffffu, T.x < 1e-4f && T.y < 1e-4f)) break;
+          if (__all_sync(0xffffffffu, saturated())) break;
         }
       };
       // The entries of this warp's block in list order: the whole batch, or
       // (CKPT) 32 at a time, the shortest segment.
       uint32_t cnt = 0;
-      const bool live = !__all_sync(0xffffffffu, T.x < 1e-4f && T.y < 1e-4f);
+      const bool live = !__all_sync(0xffffffffu, saturated());
       for (uint32_t base = 0; (CKPT || live) && base < nb; base += 32) {
         const uint32_t j = base + lane;
         const bool bit = j < nb && ((s_mask[j] >> warp) & 1u);
@@ -520,14 +600,15 @@ __global__ void __launch_bounds__(TW* TH / 2, CKPT ? 4 : kFwdThreadsPerSm / (TW 
         if (bit) list[cnt + __popc(bal & ((1u << lane) - 1u))] = (uint16_t)(j * sizeof(FwdEntry));
         cnt += __popc(bal);
         if constexpr (CKPT) {
-          if (cnt && !__all_sync(0xffffffffu, T.x < 1e-4f && T.y < 1e-4f)) walk(cnt);
+          if (cnt && !__all_sync(0xffffffffu, saturated())) walk(cnt);
           cnt = 0;
           __syncwarp();  // the list is free again
           if ((stored + 1) * seg_len == b0 - s0 + base + 32 && stored + 1 < a.b.seg_k) {  // the last one is open-ended
             float4* c = ck + (size_t)stored * (TW * TH);
-            c[0] = make_float4(T.x, S0.x, S1.x, S2.x);
-            c[NT] = make_float4(T.y, S0.y, S1.y, S2.y);
-            S0 = S1 = S2 = f2(0.f);
+#pragma unroll
+            for (int h = 0; h < PX; ++h)
+              c[h * kHalf] = make_float4(L::get(T, h), L::get(S0, h), L::get(S1, h), L::get(S2, h));
+            S0 = S1 = S2 = L::all(0.f);
             ++stored;
           }
         }
@@ -536,45 +617,76 @@ __global__ void __launch_bounds__(TW* TH / 2, CKPT ? 4 : kFwdThreadsPerSm / (TW 
       __syncthreads();
       for (uint32_t j = threadIdx.x; j < nb; j += NT) {
         const uint32_t h = *reinterpret_cast<const uint32_t*>(s_e[j].hit);
-        hitw[b0 + j] = (uint8_t)((h | (h >> 7) | (h >> 14) | (h >> 21)) & 0xfu);  // bit w: the 8x8 block of warp w
+        if (SPLIT) {
+          // The other blocks' CTAs set their bits in the same byte.
+          const uintptr_t at = reinterpret_cast<uintptr_t>(hitw + b0 + j);
+          if (h) atomicOr(reinterpret_cast<uint32_t*>(at & ~uintptr_t(3)), (1u << block) << (8 * (at & 3)));
+        } else {
+          hitw[b0 + j] = (uint8_t)((h | (h >> 7) | (h >> 14) | (h >> 21)) & 0xfu);  // bit w: the 8x8 block of warp w
+        }
         if (h) vis[s_e[j].cidx] = 1;
       }
-      if (__syncthreads_and(T.x < 1e-4f && T.y < 1e-4f)) break;
+      if (__syncthreads_and(saturated())) break;
     }
     if constexpr (CKPT) {
       // Each thread turns its own checkpoints' colours into the sum over the
       // later segments, from the last one forward.
       for (int k = (int)stored - 1; k >= 0; --k) {
         float4* c = ck + (size_t)k * (TW * TH);
-        const float4 u = c[0], w = c[NT];
-        c[0] = make_float4(u.x, S0.x, S1.x, S2.x);
-        c[NT] = make_float4(w.x, S0.y, S1.y, S2.y);
-        S0 = add2(S0, make_float2(u.y, w.y));
-        S1 = add2(S1, make_float2(u.z, w.z));
-        S2 = add2(S2, make_float2(u.w, w.w));
+        float c0[PX], c1[PX], c2[PX];
+#pragma unroll
+        for (int h = 0; h < PX; ++h) {
+          const float4 u = c[h * kHalf];
+          c[h * kHalf] = make_float4(u.x, L::get(S0, h), L::get(S1, h), L::get(S2, h));
+          c0[h] = u.y;
+          c1[h] = u.z;
+          c2[h] = u.w;
+        }
+        S0 = add2(S0, L::make(c0));
+        S1 = add2(S1, L::make(c1));
+        S2 = add2(S2, L::make(c2));
       }
     }
     float4* out = reinterpret_cast<float4*>(a.out_rgba) + vd.pix_base;
-    auto finish = [&](uint32_t row, float Tq, float c0, float c1, float c2, uint32_t last, uint32_t nc) {
-      const size_t pix = (size_t)row * vd.w + px;
-      out[pix] = make_float4(c0 + Tq * a.bg[0], c1 + Tq * a.bg[1], c2 + Tq * a.bg[2], 1.f - Tq);
+    uint32_t ml = 0;
+#pragma unroll
+    for (int h = 0; h < PX; ++h) {
+      ml = max(ml, last[h]);
+      if (!inside[h]) continue;
+      const size_t pix = (size_t)(py + 4 * h) * vd.w + px;
+      const float Tq = L::get(T, h);
+      out[pix] = make_float4(L::get(C0, h) + Tq * a.bg[0], L::get(C1, h) + Tq * a.bg[1], L::get(C2, h) + Tq * a.bg[2],
+                             1.f - Tq);
       slice(a.b.tfinal, a.b.Pcap, v)[pix] = Tq;
-      slice(a.b.last, a.b.Pcap, v)[pix] = last;
-      slice(a.b.ncontrib, a.b.Pcap, v)[pix] = nc;
-      slice(a.b.nvisit, a.b.Pcap, v)[pix] = (Tq < 1e-4f ? last : s1) - s0;  // a saturated pixel stopped there
-    };
-    if (in0) finish(py, T.x, C0.x, C1.x, C2.x, last0, nc0);
-    if (in1) finish(py + 4, T.y, C0.y, C1.y, C2.y, last1, nc1);
+      slice(a.b.last, a.b.Pcap, v)[pix] = last[h];
+      slice(a.b.ncontrib, a.b.Pcap, v)[pix] = nc[h];
+      slice(a.b.nvisit, a.b.Pcap, v)[pix] = (Tq < 1e-4f ? last[h] : s1) - s0;  // a saturated pixel stopped there
+    }
     // The backward's cost of this item: list entries up to the tile's
     // largest last contributor.
-    const uint32_t ml = __reduce_max_sync(0xffffffffu, max(last0, last1));
+    ml = __reduce_max_sync(0xffffffffu, ml);
     if (lane == 0 && ml) atomicMax(&s_work, ml);
     __syncthreads();
-    const uint32_t cost = s_work > s0 ? s_work - s0 : 0u;
-    const uint32_t nseg = CKPT ? min(a.b.seg_k, max((cost + seg_len - 1u) / seg_len, 1u)) : 1u;
-    for (uint32_t g = threadIdx.x; g < nseg; g += NT) {  // the tile's backward items, one per segment
-      const uint32_t k = cost_bucket(g + 1 < nseg ? seg_len : cost - g * seg_len);
-      a.b.sched_lists[(size_t)k * a.b.sched_items_cap + atomicAdd(a.b.sched_lcount + k, 1u)] = item * a.b.seg_k + g;
+    uint32_t top = s_work;
+    if (SPLIT) {
+      // The last of the tile's four CTAs knows the tile's.
+      __shared__ uint32_t s_top;
+      if (threadIdx.x == 0) {
+        uint32_t* sync = a.b.tile_sync + 2 * (size_t)item;
+        atomicMax(sync, top);
+        __threadfence();
+        s_top = atomicAdd(sync + 1, 1u) == 3u ? atomicMax(sync, 0u) : 0xffffffffu;
+      }
+      __syncthreads();
+      top = s_top;
+    }
+    if (!SPLIT || top != 0xffffffffu) {
+      const uint32_t cost = top > s0 ? top - s0 : 0u;
+      const uint32_t nseg = CKPT ? min(a.b.seg_k, max((cost + seg_len - 1u) / seg_len, 1u)) : 1u;
+      for (uint32_t g = threadIdx.x; g < nseg; g += NT) {  // the tile's backward items, one per segment
+        const uint32_t c = cost_bucket(g + 1 < nseg ? seg_len : cost - g * seg_len);
+        a.b.sched_lists[(size_t)c * a.b.sched_items_cap + atomicAdd(a.b.sched_lcount + c, 1u)] = item * a.b.seg_k + g;
+      }
     }
     __syncthreads();
     if (threadIdx.x == 0) s_work = 0u;
@@ -1293,6 +1405,19 @@ __global__ void __launch_bounds__(32, kTileBwdBlocks) raster_bwd_tile_kernel(Ras
   }
 }
 
+// A split forward's CTAs set the hit bits of their blocks one by one.
+__global__ void __launch_bounds__(256) zero_hits_kernel(FwdBufs b) {
+  const uint32_t v = blockIdx.y, n = b.vcount[v * 4 + 1];
+  uint8_t* hitw = slice(b.hitw, b.Icap, v);
+  // Whole 16-byte words and the ragged ends.
+  const uint32_t head = min(n, (uint32_t)(-reinterpret_cast<uintptr_t>(hitw) & 15)), words = (n - head) / 16;
+  const uint32_t i0 = blockIdx.x * 256 + threadIdx.x;
+  uint4* mid = reinterpret_cast<uint4*>(hitw + head);
+  for (uint32_t i = i0; i < words; i += gridDim.x * 256) mid[i] = make_uint4(0, 0, 0, 0);
+  if (i0 < head) hitw[i0] = 0;
+  if (i0 < n - head - words * 16) hitw[head + words * 16 + i0] = 0;
+}
+
 // Deterministic mode: zero partial sums for every intersection; the backward
 // then writes those of the entries that some pixel took. Most list entries
 // lie behind saturated pixels, and a warp per tile clearing its own list's
@@ -1344,25 +1469,27 @@ cudaError_t launch_items(int threads, const RasterArgs& a, uint32_t items, int n
   return cudaGetLastError();
 }
 
-template <int TW, int TH, int BATCH, bool CKPT>
+template <int TW, int TH, int BATCH, bool CKPT, bool SPLIT>
 cudaError_t launch_fwd_batch(const RasterArgs& a, int num_sms, cudaStream_t st) {
-  return launch_items<raster_fwd_kernel<TW, TH, BATCH, CKPT>>(TW * TH / 2, a, a.vs.total_tiles, num_sms, st);
+  return launch_items<raster_fwd_kernel<TW, TH, BATCH, CKPT, SPLIT>>(SPLIT ? 64 : TW * TH / 2, a,
+                                                                     a.vs.total_tiles * (SPLIT ? 4 : 1), num_sms, st);
 }
 template <int TW, int TH>
 cudaError_t launch_fwd_shape(const RasterArgs& a, uint32_t batch, int num_sms, cudaStream_t st) {
   switch (pick_batch(batch, 128)) {
-    case 64: return launch_fwd_batch<TW, TH, 64, false>(a, num_sms, st);
-    case 128: return launch_fwd_batch<TW, TH, 128, false>(a, num_sms, st);
-    default: return launch_fwd_batch<TW, TH, 256, false>(a, num_sms, st);
+    case 64: return launch_fwd_batch<TW, TH, 64, false, false>(a, num_sms, st);
+    case 128: return launch_fwd_batch<TW, TH, 128, false, false>(a, num_sms, st);
+    default: return launch_fwd_batch<TW, TH, 256, false, false>(a, num_sms, st);
   }
 }
 // 16x16 tiles: with checkpoints when the backward is segmented.
 cudaError_t launch_fwd_16(const RasterArgs& a, uint32_t batch, int num_sms, cudaStream_t st) {
   if (a.b.seg_k == 1) return launch_fwd_shape<16, 16>(a, batch, num_sms, st);
+  if (a.split) return launch_fwd_batch<16, 16, 64, true, true>(a, num_sms, st);
   switch (pick_batch(batch, 64)) {
-    case 64: return launch_fwd_batch<16, 16, 64, true>(a, num_sms, st);
-    case 128: return launch_fwd_batch<16, 16, 128, true>(a, num_sms, st);
-    default: return launch_fwd_batch<16, 16, 256, true>(a, num_sms, st);
+    case 64: return launch_fwd_batch<16, 16, 64, true, false>(a, num_sms, st);
+    case 128: return launch_fwd_batch<16, 16, 128, true, false>(a, num_sms, st);
+    default: return launch_fwd_batch<16, 16, 256, true, false>(a, num_sms, st);
   }
 }
 template <int TW, int TH, int PPL, bool REF>
@@ -1426,7 +1553,7 @@ void raster_warm_up(uint32_t tile_w, uint32_t tile_h, uint32_t batch, int num_sm
       (void)launch_fwd_16(a, batch, num_sms, nullptr);
       (void)launch_bwd_16(a, num_sms, nullptr);
       a.b.seg_k = 2;
-      (void)launch_fwd_16(a, batch, num_sms, nullptr);
+      for (a.split = 0; a.split < 2; ++a.split) (void)launch_fwd_16(a, batch, num_sms, nullptr);
       (void)launch_bwd_16(a, num_sms, nullptr);
     } else if (tile_w == 8 && tile_h == 8) {
       (void)launch_fwd_shape<8, 8>(a, batch, num_sms, nullptr);
@@ -1451,9 +1578,18 @@ cudaError_t launch_raster_fwd(const ViewSet& vs, FwdBufs& b, const float* bg, fl
   cudaError_t e = cudaMemsetAsync(b.visible_c, 0, b.Vcap * vs.n_views, st);
   if (e != cudaSuccess) return e;
   if (vs.total_tiles == 0) return cudaSuccess;
-  // The forward appends every item to the cost list of its backward cost.
-  e = cudaMemsetAsync(b.sched_lcount, 0, sizeof(uint32_t) * kCostLists, st);
+  a.split = vs.tile_w == 16 && vs.tile_h == 16 && vs.total_tiles <= kFwdSplitTiles &&
+            (uint64_t)vs.n_splats >= (uint64_t)kFwdSplitSplats * vs.total_tiles;
+  // The forward appends every item to the cost list of its backward cost; the
+  // CTAs of a split tile meet in tile_sync, which follows the lists' counts.
+  static_assert(kFwdSplitTiles <= kSegItems / 4, "split tiles leave checkpoints");
+  e = cudaMemsetAsync(b.sched_lcount, 0, sizeof(uint32_t) * (kCostLists + (a.split ? 2 * vs.total_tiles : 0)), st);
   if (e != cudaSuccess) return e;
+  if (a.split) {
+    zero_hits_kernel<<<dim3(std::max(1, s.num_sms * 2 / (int)vs.n_views), vs.n_views), 256, 0, st>>>(b);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
   a.persist = (vs.persistent & kPersistFwd) != 0 ? 1 : 0;
   if (a.persist) {
     sched_order_kernel<<<1, kOrderThreads, 0, st>>>(vs, b);

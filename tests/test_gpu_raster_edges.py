@@ -59,3 +59,33 @@ def test_list_lengths(gsr_ctx_factory, n, kind):
     od = oracle_forward(sc, sc.cameras[0], f64=True).backward(up, mode=0)
     for k in ("v_transforms", "v_sh", "v_raw_opacity"):
         assert_grad_parity(got[k].cpu().numpy(), ob[k], od[k], what=k)
+
+
+@pytest.mark.parametrize("schedule", ["default", "grid", "persistent"])
+@pytest.mark.parametrize("n,w,h", [(700, 33, 31), (3000, 16, 40), (40_000, 512, 500), (32_767, 512, 512),
+                                   (40_000, 513, 512)])
+def test_split_tiles(gsr_ctx_factory, n, w, h, schedule):
+    """Launches around the line where each 8x8 block is blended in a CTA of its
+    own (1024 tiles, 32 Gaussians a tile), with partial tiles, in every
+    schedule and with an odd view capacity, so that the views' hit bits start
+    at odd addresses."""
+    import torch
+
+    from rustscan_b200 import host_splats_to_device
+
+    sc = _scene(n, "dots", w, h)
+    cams = sc.cameras if w * h > 4000 else sc.cameras * 3
+    ctx = gsr_ctx_factory(max_splats=n, max_views=len(cams), max_pixels=w * h, max_isects=400_003, schedule=schedule)
+    splats = host_splats_to_device(sc)
+    _, g = run_gpu_forward(ctx, splats, cams)
+    o = oracle_forward(sc, cams[0])
+    for view in g:
+        assert_forward_parity(view, o)
+    up = S.upstream_grad(h, w, seed=n)
+    v = torch.as_tensor(np.concatenate([up.reshape(-1)] * len(cams)), device="cuda")
+    got = ctx.render_backward(splats, v)
+    torch.cuda.synchronize()
+    ob = o.backward(up, mode=0)
+    od = oracle_forward(sc, cams[0], f64=True).backward(up, mode=0)
+    for k in ("v_transforms", "v_sh", "v_raw_opacity"):
+        assert_grad_parity(got[k].cpu().numpy() / len(cams), ob[k], od[k], what=k)
