@@ -385,7 +385,9 @@ GSR_API gsr_status gsr_autotune(const gsr_config* base, const gsr_splats* splats
  * capture). gsr_profile_read synchronises the stream and writes the
  * milliseconds per stage, summed since the last read, in this order:
  * project, depth_sort, offsets, emit, tile_sort, ranges, raster_fwd,
- * visible, loss, raster_bwd, reduce, project_bwd, adam (13 entries). */
+ * visible, loss, raster_bwd, reduce, project_bwd (in a training step with
+ * Adam), adam (13 entries; with few Gaussians the depth sort is part of
+ * offsets). */
 enum { GSR_PROFILE_STAGES = 13 };
 GSR_API gsr_status gsr_profile(gsr_ctx* ctx, int32_t enable);
 GSR_API gsr_status gsr_profile_read(gsr_ctx* ctx, float* ms_per_stage, int32_t n_stages, void* stream);

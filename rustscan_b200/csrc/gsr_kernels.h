@@ -40,7 +40,6 @@ struct FwdBufs {
   uint32_t* blk_base;      // projection: [views][proj_parts_cap] exclusive scan of blk_count
   uint32_t proj_parts_cap;
   float4* sgrad;           // [V][3] screen-space gradient sums (12 floats)
-  float4* pair;            // [views][6][Vcap]: six float4 planes of projection adjoint records
   float* sgrad_part;       // [I][12] per-intersection partial sums (deterministic mode)
   uint32_t* inv_perm;      // [I] emission index -> sorted position (deterministic mode)
   uint32_t* vcount;        // [4] visible, intersections (clamped), intersections required, pad
@@ -266,9 +265,10 @@ struct AdamArgs {
 cudaError_t launch_set_scalars(AdamScalars* dst, const AdamScalars& v, cudaStream_t st);
 
 // Project backward over all Gaussians for all views of the last forward:
-// writes the gradients (summed over views, scaled by grad_scale), optional
-// per-view stats, and optionally accumulates the densification statistics
-// view by view.
+// writes the gradients (summed over views, scaled by grad_scale) or, with adam,
+// updates the parameters and moments with them (sp's arrays are then adam's);
+// optional per-view stats, and optionally accumulates the densification
+// statistics view by view.
 struct ProjBwdArgs {
   float* v_tr;
   float* v_sh;
@@ -279,6 +279,7 @@ struct ProjBwdArgs {
   float grad_scale;
   int exact;
   int hp;  // FP64 conic mode of the forward
+  const AdamArgs* adam;  // host pointer, null: write the gradients
 };
 cudaError_t launch_project_bwd(const SplatsDev& sp, const ViewSet& vs, float cov_blur, FwdBufs& b,
                                const ProjBwdArgs& a, cudaStream_t st, int num_sms);
