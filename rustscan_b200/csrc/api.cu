@@ -158,7 +158,7 @@ gsr_status allocate(gsr_ctx* c) {
             dalloc(c, &b.ncontrib, nv * P) && dalloc(c, &b.nvisit, nv * P) && dalloc(c, &b.visible_c, nv * V) &&
             dalloc(c, &b.sgrad, nv * V * 3) && dalloc(c, &b.vcount, nv * 4) &&
             dalloc(c, &b.tile_hist, nv * T) && dalloc(c, &b.hitw, nv * I + 4) && dalloc(c, &b.sched_order, nv * T) &&
-            dalloc(c, &b.sched_lcount, 32 + 2 * kFwdSplitTiles) && dalloc(c, &b.sched_ticket, 1);
+            dalloc(c, &b.sched_lcount, kSchedWords) && dalloc(c, &b.sched_ticket, 1);
   b.tile_sync = b.sched_lcount + 32;
   // Backward work items: the tiles, or the segments of a launch of few tiles.
   b.sched_items_cap = std::max<uint64_t>(nv * T, kSegItems);
@@ -198,7 +198,7 @@ gsr_status allocate(gsr_ctx* c) {
       cudaMemset(c->s.ctl, 0, sizeof(LookbackCtl)) != cudaSuccess ||
       cudaMemset(c->s.status, 0, sizeof(DevStatus)) != cudaSuccess ||
       cudaMemset(b.vcount, 0, sizeof(uint32_t) * 4 * nv) != cudaSuccess ||
-      cudaMemset(b.sched_lcount, 0, sizeof(uint32_t) * 32) != cudaSuccess)
+      cudaMemset(b.sched_lcount, 0, sizeof(uint32_t) * kSchedWords) != cudaSuccess)
     return cuda_fail(c, cudaGetLastError(), "cudaMemset");
   raster_warm_up(cfg.tile_w, cfg.tile_h, cfg.batch, c->num_sms);
   return GSR_OK;
@@ -303,11 +303,10 @@ gsr_status forward_impl(gsr_ctx* c, const gsr_splats* sp, const gsr_camera* cams
   rs = build_views(c, cams, n_views, desc, vs);
   if (rs != GSR_OK) return rs;
   vs.n_splats = sp->n;
-  GSR_CUDA(c, launch_set_views(c->d_views, desc.data(), n_views, st));
   const SplatsDev sd = splats_dev(c, sp);
   FwdBufs& b = c->b;
   prof_mark(c, kStProject, st);
-  GSR_CUDA(c, launch_project(sd, vs, c->cfg.cov_blur, c->cfg.fp64_conic, b, c->s, st));
+  GSR_CUDA(c, launch_project(sd, vs, desc.data(), c->d_views, c->cfg.cov_blur, c->cfg.fp64_conic, b, st));
   prof_mark(c, kStDepthSort, st);
   // Few Gaussians: one cluster per view sorts and scans at once, below.
   const bool one_launch = order_fits_cluster(sp->n, n_views, c->s);

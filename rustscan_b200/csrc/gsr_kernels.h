@@ -86,6 +86,8 @@ constexpr uint32_t kSegItems = 16384, kSegMax = 64;
 // 50k 101 and 78, 900 over 120k 100 and 92, 1024 over 200k 117 and 108, 1200
 // over 200k 100 and 100, 2025 over 300k 124 and 132; 1024 over 10k 33 and 37.
 constexpr uint32_t kFwdSplitTiles = 1024, kFwdSplitSplats = 32;
+// Words of sched_lcount with tile_sync behind it.
+constexpr uint32_t kSchedWords = 32 + 2 * kFwdSplitTiles;
 
 // Bits of ViewSet::persistent (otherwise one CTA per work item).
 constexpr int kPersistFwd = 1, kPersistBwd = 2;
@@ -122,8 +124,11 @@ struct Scratch {
 constexpr uint32_t kProjBlock = 256;
 
 // ---- launchers (return cudaGetLastError()) ----
-cudaError_t launch_project(const SplatsDev& sp, const ViewSet& vs, float cov_blur, int fp64_conic, FwdBufs& b,
-                           const Scratch& s, cudaStream_t st);
+// Projects, compacts and colours all views; also writes the view descriptors
+// (host_views) to dev_views and clears tile_hist, sched_lcount with tile_sync,
+// and visible_c.
+cudaError_t launch_project(const SplatsDev& sp, const ViewSet& vs, const ViewDesc* host_views, ViewDesc* dev_views,
+                           float cov_blur, int fp64_conic, FwdBufs& b, cudaStream_t st);
 
 // Stable LSD radix sort of (key, value) pairs in `segments` segments of
 // seg_stride elements; segment i holds counts[i * count_stride] elements

@@ -402,8 +402,7 @@ cudaError_t launch_emit_hist(const ViewSet& vs, FwdBufs& b, const Scratch& s, in
                              cudaStream_t st) {
   if (vs.max_tiles > kHistMaxTiles) return cudaErrorInvalidValue;
   if (slots && deterministic) return cudaErrorInvalidValue;
-  cudaError_t e = cudaMemsetAsync(b.tile_hist, 0, sizeof(uint32_t) * b.Tcap * vs.n_views, st);
-  if (e != cudaSuccess) return e;
+  cudaError_t e;
   const size_t smem = sizeof(uint32_t) * vs.max_tiles;
   // The per-tile counts may take the static walk state past the 48 KB
   // default: allow the largest histogram.

@@ -1575,16 +1575,13 @@ cudaError_t launch_raster_fwd(const ViewSet& vs, FwdBufs& b, const float* bg, fl
   a.bg[1] = bg[1];
   a.bg[2] = bg[2];
   a.out_rgba = out_rgba;
-  cudaError_t e = cudaMemsetAsync(b.visible_c, 0, b.Vcap * vs.n_views, st);
-  if (e != cudaSuccess) return e;
+  cudaError_t e;
   if (vs.total_tiles == 0) return cudaSuccess;
   a.split = vs.tile_w == 16 && vs.tile_h == 16 && vs.total_tiles <= kFwdSplitTiles &&
             (uint64_t)vs.n_splats >= (uint64_t)kFwdSplitSplats * vs.total_tiles;
-  // The forward appends every item to the cost list of its backward cost; the
-  // CTAs of a split tile meet in tile_sync, which follows the lists' counts.
+  // The CTAs of a split tile leave checkpoints and meet in tile_sync, which the
+  // projection cleared, as it did the cost lists' counts.
   static_assert(kFwdSplitTiles <= kSegItems / 4, "split tiles leave checkpoints");
-  e = cudaMemsetAsync(b.sched_lcount, 0, sizeof(uint32_t) * (kCostLists + (a.split ? 2 * vs.total_tiles : 0)), st);
-  if (e != cudaSuccess) return e;
   if (a.split) {
     zero_hits_kernel<<<dim3(std::max(1, s.num_sms * 2 / (int)vs.n_views), vs.n_views), 256, 0, st>>>(b);
     e = cudaGetLastError();
