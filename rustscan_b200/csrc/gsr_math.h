@@ -276,15 +276,23 @@ template <class F> GSR_HD M3<F> rot_scale(const M3<F>& r, V3<F> s) {
   return m;
 }
 
-// helpers.wgsl:138-154. The limits follow the WGSL expression exactly.
-template <class F> GSR_HD M32<F> calc_cam_j(V3<F> mc, const Cam<F>& c) {
-  const F limx_pos = (F(1.15) * F(c.w) - c.pc.x) / c.focal.x;
-  const F limy_pos = (F(1.15) * F(c.h) - c.pc.y) / c.focal.y;
-  const F limx_neg = (F(-0.15) * F(c.w) - c.pc.x) / c.focal.x;
-  const F limy_neg = (F(-0.15) * F(c.h) - c.pc.y) / c.focal.y;
-  const F rz = F(1) / gmax(mc.z, F(0.01));
-  const F u = clampf(mc.x * rz, limx_neg, limx_pos);
-  const F v = clampf(mc.y * rz, limy_neg, limy_pos);
+// helpers.wgsl:138-154. The limits follow the WGSL expression exactly; they
+// depend on the view alone.
+template <class F> struct CamLimits {
+  F x_neg, x_pos, y_neg, y_pos;
+};
+template <class F> GSR_HD CamLimits<F> cam_limits(const Cam<F>& c) {
+  CamLimits<F> l;
+  l.x_pos = (F(1.15) * F(c.w) - c.pc.x) / c.focal.x;
+  l.y_pos = (F(1.15) * F(c.h) - c.pc.y) / c.focal.y;
+  l.x_neg = (F(-0.15) * F(c.w) - c.pc.x) / c.focal.x;
+  l.y_neg = (F(-0.15) * F(c.h) - c.pc.y) / c.focal.y;
+  return l;
+}
+// rz = 1 / max(mc.z, 0.01).
+template <class F> GSR_HD M32<F> calc_cam_j(V3<F> mc, F rz, const CamLimits<F>& l, const Cam<F>& c) {
+  const F u = clampf(mc.x * rz, l.x_neg, l.x_pos);
+  const F v = clampf(mc.y * rz, l.y_neg, l.y_pos);
   const F dx = c.focal.x * rz, dy = c.focal.y * rz;
   M32<F> j;
   j.m[0][0] = dx;
@@ -294,6 +302,9 @@ template <class F> GSR_HD M32<F> calc_cam_j(V3<F> mc, const Cam<F>& c) {
   j.m[2][0] = -dx * u;
   j.m[2][1] = -dy * v;
   return j;
+}
+template <class F> GSR_HD M32<F> calc_cam_j(V3<F> mc, const Cam<F>& c) {
+  return calc_cam_j(mc, F(1) / gmax(mc.z, F(0.01)), cam_limits(c), c);
 }
 
 // helpers.wgsl:170-183. Returns the opacity compensation and adds the blur.
@@ -376,11 +387,13 @@ struct TileBox {
   uint32_t x0, y0, x1, y1;  // [x0, x1) x [y0, y1) in tile units
 };
 
-// helpers.wgsl:204-216 generalised to tw x th tiles.
+// helpers.wgsl:204-216 generalised to tw x th tiles. inv_tile holds the
+// reciprocals of the tile's sides: they are powers of two, so the products
+// round as the quotients do.
 template <class F>
-GSR_HD TileBox tile_bbox(V2<F> center, V2<F> ext, TileShape ts, uint32_t tiles_x, uint32_t tiles_y) {
-  const F cx = center.x / F(ts.tw), cy = center.y / F(ts.th);
-  const F ex = ext.x / F(ts.tw), ey = ext.y / F(ts.th);
+GSR_HD TileBox tile_bbox(V2<F> center, V2<F> ext, V2<F> inv_tile, uint32_t tiles_x, uint32_t tiles_y) {
+  const F cx = center.x * inv_tile.x, cy = center.y * inv_tile.y;
+  const F ex = ext.x * inv_tile.x, ey = ext.y * inv_tile.y;
   TileBox b;
   b.x0 = (uint32_t)clampf(cx - ex, F(0), F(tiles_x));
   b.y0 = (uint32_t)clampf(cy - ey, F(0), F(tiles_y));
@@ -603,11 +616,12 @@ GSR_HD GaussWorld<F> gauss_world(V4<F> quat, V3<F> log_scale, F raw_opac) {
   return w;
 }
 
-// project_gaussian with the view-independent part computed once (kernels
-// that project one Gaussian into many views).
+// project_gaussian with the parts of the Gaussian and of the view computed
+// once (kernels that project many Gaussians into many views).
 template <class F>
-GSR_HD Projected<F> project_gaussian_w(const Cam<F>& cam, V3<F> mean, const GaussWorld<F>& gw, F cov_blur,
-                                       TileShape ts, uint32_t tiles_x, uint32_t tiles_y, bool hp = false) {
+GSR_HD Projected<F> project_gaussian_w(const Cam<F>& cam, const CamLimits<F>& lim, V3<F> mean,
+                                       const GaussWorld<F>& gw, F cov_blur, V2<F> inv_tile, uint32_t tiles_x,
+                                       uint32_t tiles_y, bool hp = false) {
   Projected<F> p;
   p.visible = false;
   const V3<F> mc = world_to_cam(cam, mean);
@@ -616,11 +630,12 @@ GSR_HD Projected<F> project_gaussian_w(const Cam<F>& cam, V3<F> mean, const Gaus
   if (!gw.ok) return p;
   F opacity = gw.opacity;
   const M3<F> cov_cam = mul(mul(cam.rot, gw.cov3d), transpose(cam.rot));
-  const M32<F> j = calc_cam_j(mc, cam);
+  const F rz_cov = F(1) / gmax(mc.z, F(0.01));
+  const M32<F> j = calc_cam_j(mc, rz_cov, lim, cam);
   M2<F> cov2d = mul(mul(j, cov_cam), transpose(j));
   opacity = opacity * (hp ? compensate_cov2d_hp(cov2d, cov_blur) : compensate_cov2d(cov2d, cov_blur));
   if (opacity < F(1.0 / 255.0)) return p;
-  const F rz = F(1) / mc.z;
+  const F rz = mc.z >= F(0.01) ? rz_cov : mc.z;  // 1 / z: only a NaN depth comes here below 0.01
   V2<F> mean2d;
   mean2d.x = cam.focal.x * mc.x * rz + cam.pc.x;
   mean2d.y = cam.focal.y * mc.y * rz + cam.pc.y;
@@ -636,7 +651,7 @@ GSR_HD Projected<F> project_gaussian_w(const Cam<F>& cam, V3<F> mean, const Gaus
   p.conic = conic;
   p.opacity = opacity;
   p.thr = thr;
-  p.box = tile_bbox(mean2d, ext, ts, tiles_x, tiles_y);
+  p.box = tile_bbox(mean2d, ext, inv_tile, tiles_x, tiles_y);
   return p;
 }
 
@@ -644,7 +659,9 @@ template <class F>
 GSR_HD Projected<F> project_gaussian(const Cam<F>& cam, V3<F> mean, V4<F> quat, V3<F> log_scale, F raw_opac,
                                      F cov_blur, TileShape ts, uint32_t tiles_x, uint32_t tiles_y,
                                      bool hp = false) {
-  return project_gaussian_w(cam, mean, gauss_world(quat, log_scale, raw_opac), cov_blur, ts, tiles_x, tiles_y, hp);
+  const V2<F> inv_tile{F(1) / F(ts.tw), F(1) / F(ts.th)};
+  return project_gaussian_w(cam, cam_limits(cam), mean, gauss_world(quat, log_scale, raw_opac), cov_blur, inv_tile,
+                            tiles_x, tiles_y, hp);
 }
 
 // Number of tiles of the box that pass the contribution test, visited in
