@@ -161,7 +161,7 @@ gsr_status allocate(gsr_ctx* c) {
             dalloc(c, &b.sched_lcount, kSchedWords) && dalloc(c, &b.sched_ticket, 1);
   b.tile_sync = b.sched_lcount + 32;
   // Backward work items: the tiles, or the segments of a launch of few tiles.
-  b.sched_items_cap = std::max<uint64_t>(nv * T, kSegItems);
+  b.sched_items_cap = std::max<uint64_t>(nv * T + 3 * kLongTiles, kSegItems);
   ok = ok && dalloc(c, &b.sched_lists, 32 * b.sched_items_cap);
   b.seg_k = 1;
   b.ckpt = nullptr;
@@ -359,7 +359,7 @@ gsr_status forward_impl(gsr_ctx* c, const gsr_splats* sp, const gsr_camera* cams
   prof_mark(c, kStRanges, st);
   if (!tile_counts) GSR_CUDA(c, launch_ranges(vs, b, c->s, st));
   prof_mark(c, kStRasterFwd, st);
-  GSR_CUDA(c, launch_raster_fwd(vs, b, c->cfg.background, out_rgba, c->s, st));
+  GSR_CUDA(c, launch_raster_fwd(vs, b, c->cfg.background, out_rgba, c->cfg.deterministic, c->s, st));
   prof_mark(c, kStVisible, st);
   if (out_visible) GSR_CUDA(c, launch_visible_out(vs, b, sp->n, out_visible, st));
   c->have_fwd = true;

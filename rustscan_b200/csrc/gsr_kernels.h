@@ -86,6 +86,18 @@ constexpr uint32_t kSegItems = 16384, kSegMax = 64;
 // 50k 101 and 78, 900 over 120k 100 and 92, 1024 over 200k 117 and 108, 1200
 // over 200k 100 and 100, 2025 over 300k 124 and 132; 1024 over 10k 33 and 37.
 constexpr uint32_t kFwdSplitTiles = 1024, kFwdSplitSplats = 32;
+// Launches of many tiles, whose backward walks a tile's list in one piece: a
+// tile that gets through more than kLongTile entries (views of few pixels beside
+// large ones) would outlast all others, so its four 8x8 blocks become items of
+// their own: each walks the entries that reach the block, up to the block's last
+// contributor, and their sums meet in the atomic adds that tiles' sums meet in.
+// At most kLongTiles of them a launch, and none in deterministic mode. Backward of
+// 16 uneven views of up to 1280x720, 500k Gaussians (longest walk 28630) 2.87 ->
+// 1.84 ms, 5 of up to 960x540, 300k (15609) 1.79 -> 1.08, 8 of up to 1200x700, 800k
+// 2.67 -> 1.66; 16 of up to 1920x1080, 2M (18429, hidden behind the other tiles)
+// 2.92 both, where the blocks' extra reductions cost 2% from 1024 entries and 0.6%
+// from 2048; from 8192 on the second case takes 1.29.
+constexpr uint32_t kLongTile = 4096, kLongTiles = 4096;
 // Words of sched_lcount with tile_sync behind it.
 constexpr uint32_t kSchedWords = 32 + 2 * kFwdSplitTiles;
 
@@ -220,8 +232,8 @@ cudaError_t launch_ranges(const ViewSet& vs, FwdBufs& b, const Scratch& s, cudaS
 // Looks up the residency of the raster kernels of a tile shape and batch
 // (persistent schedule) outside any stream capture; enqueues nothing.
 void raster_warm_up(uint32_t tile_w, uint32_t tile_h, uint32_t batch, int num_sms);
-cudaError_t launch_raster_fwd(const ViewSet& vs, FwdBufs& b, const float* bg, float* out_rgba, const Scratch& s,
-                              cudaStream_t st);
+cudaError_t launch_raster_fwd(const ViewSet& vs, FwdBufs& b, const float* bg, float* out_rgba, int deterministic,
+                              const Scratch& s, cudaStream_t st);
 cudaError_t launch_raster_bwd(const ViewSet& vs, FwdBufs& b, const float* bg, const float* v_rgba, int ref_mode,
                               int deterministic, const Scratch& s, cudaStream_t st);
 cudaError_t launch_reduce_det(const ViewSet& vs, FwdBufs& b, const Scratch& s, cudaStream_t st);

@@ -73,6 +73,7 @@ struct RasterArgs {
   const float* v_rgba;
   int ref_mode;
   int det;
+  int long_tiles;  // forward: tiles of long lists are listed as an item per 8x8 block (see kLongTile)
   int split;    // forward: a CTA per 8x8 block of a 16x16 tile
   int persist;  // 0: one CTA per item; 1: persistent, items from sched_order; 2: persistent, items from the cost lists
 };
@@ -86,6 +87,10 @@ __device__ __forceinline__ uint32_t find_view(const ViewSet& vs, uint32_t item) 
 
 constexpr uint32_t kNoItem = 0xffffffffu;
 
+// Backward items of 16x16 tiles: the tile, and above kBlockShift which of its 8x8
+// blocks the item takes (0: all). A launch has fewer than 2^28 tiles, each with
+// 8 KB of pixel state.
+constexpr uint32_t kBlockShift = 28;
 constexpr int kCostLists = 32;  // bit lengths 0..31 of a cost (a list is shorter than 2^30); one per lane
 
 __device__ __forceinline__ uint32_t cost_bucket(uint32_t cost) { return cost ? 32u - (uint32_t)__clz(cost) : 0u; }
@@ -682,7 +687,19 @@ __global__ void __launch_bounds__(SPLIT ? 64 : TW * TH / 2, SPLIT ? 8 : CKPT ? 4
     }
     if (!SPLIT || top != 0xffffffffu) {
       const uint32_t cost = top > s0 ? top - s0 : 0u;
-      const uint32_t nseg = CKPT ? min(a.b.seg_k, max((cost + seg_len - 1u) / seg_len, 1u)) : 1u;
+      bool split = false;
+      if (!CKPT && TW == 16 && TH == 16 && a.long_tiles && cost > kLongTile) {
+        // Room for kLongTiles of them; tile_sync is free in a launch without checkpoints.
+        if (threadIdx.x == 0 && (s_item = atomicAdd(a.b.tile_sync, 1u)) < kLongTiles) {
+          const uint32_t c = cost_bucket(cost / 2);
+          const uint32_t at = atomicAdd(a.b.sched_lcount + c, 4u);
+          for (uint32_t q = 0; q < 4; ++q)
+            a.b.sched_lists[(size_t)c * a.b.sched_items_cap + at + q] = item | (q + 1) << kBlockShift;
+        }
+        __syncthreads();
+        split = s_item < kLongTiles;
+      }
+      const uint32_t nseg = split ? 0u : CKPT ? min(a.b.seg_k, max((cost + seg_len - 1u) / seg_len, 1u)) : 1u;
       for (uint32_t g = threadIdx.x; g < nseg; g += NT) {  // the tile's backward items, one per segment
         const uint32_t c = cost_bucket(g + 1 < nseg ? seg_len : cost - g * seg_len);
         a.b.sched_lists[(size_t)c * a.b.sched_items_cap + atomicAdd(a.b.sched_lcount + c, 1u)] = item * a.b.seg_k + g;
@@ -1202,7 +1219,9 @@ __global__ void __launch_bounds__(32, kTileBwdBlocks) raster_bwd_tile_kernel(Ras
   for (uint32_t round = 0;; ++round) {
     const uint32_t work = next_item<SEG>(a, round, &s_item, &s_lists);
     if (work == kNoItem) break;
-    const uint32_t item = SEG ? work / a.b.seg_k : work, seg = SEG ? work % a.b.seg_k : 0u;
+    const uint32_t item = SEG ? work / a.b.seg_k : work & ((1u << kBlockShift) - 1u), seg = SEG ? work % a.b.seg_k : 0u;
+    // The 8x8 blocks this item takes: all, or one of a long list.
+    const uint32_t blocks = SEG || work < (1u << kBlockShift) ? 0xfu : 1u << ((work >> kBlockShift) - 1u);
     const uint32_t v = find_view(a.vs, item);
     const ViewDesc& vd = a.vs.views[v];
     const uint32_t t = item - vd.tile_base;
@@ -1227,7 +1246,7 @@ __global__ void __launch_bounds__(32, kTileBwdBlocks) raster_bwd_tile_kernel(Ras
   #pragma unroll
     for (int q = 0; q < 4; ++q) {
       load_bwd_pair(a, vd, v, px0 + 8 * (q & 1), py0 + 8 * (q >> 1), pp[q]);
-      mylast = max(mylast, max(pp[q].last0, pp[q].last1));
+      if ((blocks >> q) & 1u) mylast = max(mylast, max(pp[q].last0, pp[q].last1));
       s_v[q][0][lane] = pp[q].vr;  // kept in shared memory, not registers
       s_v[q][1][lane] = pp[q].vg;
       s_v[q][2][lane] = pp[q].vb;
@@ -1257,7 +1276,7 @@ __global__ void __launch_bounds__(32, kTileBwdBlocks) raster_bwd_tile_kernel(Ras
       for (int it = 0; it < kSI; ++it) {
         const uint32_t s = lo + lane + it * NT;
         const bool ok = s < hi;
-        ph[it] = ok ? hitw[s] : 0u;
+        ph[it] = ok ? hitw[s] & blocks : 0u;
         pc[it] = ok ? (vals[s] & vmask) : 0u;
       }
     };
@@ -1565,8 +1584,8 @@ void raster_warm_up(uint32_t tile_w, uint32_t tile_h, uint32_t batch, int num_sm
   }
 }
 
-cudaError_t launch_raster_fwd(const ViewSet& vs, FwdBufs& b, const float* bg, float* out_rgba, const Scratch& s,
-                              cudaStream_t st) {
+cudaError_t launch_raster_fwd(const ViewSet& vs, FwdBufs& b, const float* bg, float* out_rgba, int deterministic,
+                              const Scratch& s, cudaStream_t st) {
   b.seg_k = pick_segments(vs);
   RasterArgs a{};
   a.vs = vs;
@@ -1575,6 +1594,7 @@ cudaError_t launch_raster_fwd(const ViewSet& vs, FwdBufs& b, const float* bg, fl
   a.bg[1] = bg[1];
   a.bg[2] = bg[2];
   a.out_rgba = out_rgba;
+  a.long_tiles = !deterministic;  // the blocks' sums of an entry meet in an atomic add
   cudaError_t e;
   if (vs.total_tiles == 0) return cudaSuccess;
   a.split = vs.tile_w == 16 && vs.tile_h == 16 && vs.total_tiles <= kFwdSplitTiles &&
