@@ -294,8 +294,12 @@ __device__ __forceinline__ void stage_sh_rows(const __nv_bfloat16* src, uint32_t
 // a training step, the Adam passes that read the gradient back: 8 views of 1M
 // Gaussians 0.817 -> 0.573 ms, 16 uneven views of 2M (BF16 SH) 2.77 -> 1.63, one
 // view of 3M (BF16, gradients out) 0.548 -> 0.386.
+// Degree 4 runs three blocks per SM at 168 registers with a few spills: 300k
+// Gaussians at 640x480, gradient and Adam, 263 us with two blocks, 223 so (the
+// separate passes took 223), 600k in 5 views 615 and 534 (603), 659k in 2 600 and
+// 492 (522).
 template <class SHT, int DEG>
-__global__ void __launch_bounds__(kGT, DEG >= 4 ? 2 : 4) gather_kernel(GatherArgs a) {
+__global__ void __launch_bounds__(kGT, DEG >= 4 ? 3 : 4) gather_kernel(GatherArgs a) {
   constexpr int K = (DEG + 1) * (DEG + 1);
   constexpr int NSH = 3 * K;
   using L = GatherSmem<K>;
