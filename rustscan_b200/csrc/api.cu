@@ -160,8 +160,9 @@ gsr_status allocate(gsr_ctx* c) {
             dalloc(c, &b.tile_hist, nv * T) && dalloc(c, &b.hitw, nv * I + 4) && dalloc(c, &b.sched_order, nv * T) &&
             dalloc(c, &b.sched_lcount, kSchedWords) && dalloc(c, &b.sched_ticket, 1);
   b.tile_sync = b.sched_lcount + 32;
+  b.long_count = b.tile_sync + 2 * kFwdSplitTiles;
   // Backward work items: the tiles, or the segments of a launch of few tiles.
-  b.sched_items_cap = std::max<uint64_t>(nv * T + 3 * kLongTiles, kSegItems);
+  b.sched_items_cap = std::max<uint64_t>(nv * T, kSegItems) + 3 * kLongTiles;
   ok = ok && dalloc(c, &b.sched_lists, 32 * b.sched_items_cap);
   b.seg_k = 1;
   b.ckpt = nullptr;

@@ -47,6 +47,7 @@ struct FwdBufs {
   uint32_t* sched_lists;   // [32][sched_items_cap] work items by the bit length of their backward cost
   uint32_t* sched_lcount;  // [32] items in each of those lists (appended by the forward)
   uint32_t* tile_sync;     // [kFwdSplitTiles][2] split forward, after sched_lcount: largest last contributor, CTAs done
+  uint32_t* long_count;    // items of long walks listed block by block
   uint32_t* sched_ticket;  // [1] next ticket a persistent raster CTA takes
   uint64_t sched_items_cap;
   float4* ckpt;            // [kSegItems][256] per (tile, segment) and pixel: transmittance after it, colour behind it
@@ -86,10 +87,9 @@ constexpr uint32_t kSegItems = 16384, kSegMax = 64;
 // 50k 101 and 78, 900 over 120k 100 and 92, 1024 over 200k 117 and 108, 1200
 // over 200k 100 and 100, 2025 over 300k 124 and 132; 1024 over 10k 33 and 37.
 constexpr uint32_t kFwdSplitTiles = 1024, kFwdSplitSplats = 32;
-// Launches of many tiles, whose backward walks a tile's list in one piece: a
-// tile that gets through more than kLongTile entries (views of few pixels beside
-// large ones) would outlast all others, so its four 8x8 blocks become items of
-// their own: each walks the entries that reach the block, up to the block's last
+// A backward item (a whole tile's list in launches of many tiles, else a segment
+// of it) of more than kLongTile entries (views of few pixels beside large ones)
+// would outlast all others, so the tile's four 8x8 blocks become items of their own: each walks the entries that reach the block, up to the block's last
 // contributor, and their sums meet in the atomic adds that tiles' sums meet in.
 // At most kLongTiles of them a launch, and none in deterministic mode. Backward of
 // 16 uneven views of up to 1280x720, 500k Gaussians (longest walk 28630) 2.87 ->
@@ -98,8 +98,8 @@ constexpr uint32_t kFwdSplitTiles = 1024, kFwdSplitSplats = 32;
 // 2.92 both, where the blocks' extra reductions cost 2% from 1024 entries and 0.6%
 // from 2048; from 8192 on the second case takes 1.29.
 constexpr uint32_t kLongTile = 4096, kLongTiles = 4096;
-// Words of sched_lcount with tile_sync behind it.
-constexpr uint32_t kSchedWords = 32 + 2 * kFwdSplitTiles;
+// Words of sched_lcount with tile_sync and long_count behind it.
+constexpr uint32_t kSchedWords = 32 + 2 * kFwdSplitTiles + 1;
 
 // Bits of ViewSet::persistent (otherwise one CTA per work item).
 constexpr int kPersistFwd = 1, kPersistBwd = 2;

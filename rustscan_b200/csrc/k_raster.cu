@@ -354,11 +354,28 @@ template <> struct Lane<1> {
   __device__ static float get(V v, int) { return v; }
 };
 
-// Entries per segment of a list of `len` entries cut into at most k segments:
-// 32 where that covers the list, else 64 (the last segment takes the rest).
-// An item of a latency-bound launch takes about 1000 cycles an entry, so
-// short segments end it sooner; more than 64 would only lengthen its tail.
-__device__ __forceinline__ uint32_t segment_len(uint32_t len, uint32_t k) { return len <= 32u * k ? 32u : 64u; }
+// The segments of a list of `len` entries: segment k begins at len (k / K)^2,
+// rounded up to the 32 entries the forward steps by, or at 32 k (64 k where that
+// does not cover the list) if that is further on, and the last one is open-ended.
+// An item of a latency-bound launch takes about 1000 cycles an entry, so short
+// segments end it sooner; most lists saturate within a fraction of their length,
+// so the early ones are short, and a list that does not ends in segments of at
+// most 2 / K of it. Every segment begins at least 32 entries after the one before.
+// With equal segments of 64 and the rest in the last one, the backward of 2 uneven
+// views up to 260x146 over 141k Gaussians (a list of 48894) took 15.7 ms and takes
+// 0.61, of 5 up to 640x400 over 500k 7.0 and 1.5, of 8 of 400x300 over 100k 0.66
+// and 0.39; of one of 639x479 over 200k 0.118 and 0.121.
+struct Segments {
+  uint32_t len;  // shortest segment
+  float grow;
+  // First entry of segment k.
+  __device__ __forceinline__ uint32_t begin(uint32_t k) const {
+    return max(k * len, ((uint32_t)(grow * (float)(k * k)) + 31u) & ~31u);
+  }
+};
+__device__ __forceinline__ Segments segments_of(uint32_t len, uint32_t k) {
+  return Segments{len <= 32u * k ? 32u : 64u, (float)len / (float)(k * k)};
+}
 
 // A list entry as the forward stages it. Values that both pixels of a pair
 // take lie twice side by side, so that a load brings them as the register
@@ -394,7 +411,7 @@ constexpr int kFwdThreadsPerSm = 768;
 // a branch each, over blocks culled by the footprint's bounding box: 8 views
 // of 1280x720 over 1M Gaussians 1.10 -> 0.83 ms (135M -> 90M warp instructions
 // a view), one view of 320x240 over 74k 0.193 -> 0.104 ms.
-// CKPT: at the end of every segment of the list (segment_len entries) the
+// CKPT: at the end of every segment of the list (see Segments) the
 // tile's pixels leave a checkpoint for the segmented backward (see
 // raster_bwd_tile_kernel): the transmittance there and the colour the segment
 // added, turned into the colour of all later segments once the tile is done.
@@ -475,7 +492,8 @@ __global__ void __launch_bounds__(SPLIT ? 64 : TW * TH / 2, SPLIT ? 8 : CKPT ? 4
     float4* ck = CKPT ? a.b.ckpt + (size_t)item * a.b.seg_k * (TW * TH) + half * kHalf + block * 32 + lane : nullptr;
     V S0 = C0, S1 = C0, S2 = C0;  // colour added since the last checkpoint
     uint32_t stored = 0;                              // checkpoints written
-    const uint32_t seg_len = segment_len(s1 - s0, a.b.seg_k);
+    const Segments segs = segments_of(s1 - s0, CKPT ? a.b.seg_k : 1u);
+    uint32_t seg_end = s0 + segs.begin(1);
     struct Raw {
       uint32_t c;
       float4 r0, r1, r2;
@@ -608,13 +626,14 @@ __global__ void __launch_bounds__(SPLIT ? 64 : TW * TH / 2, SPLIT ? 8 : CKPT ? 4
           if (cnt && !__all_sync(0xffffffffu, saturated())) walk(cnt);
           cnt = 0;
           __syncwarp();  // the list is free again
-          if ((stored + 1) * seg_len == b0 - s0 + base + 32 && stored + 1 < a.b.seg_k) {  // the last one is open-ended
+          if (b0 + base + 32 == seg_end) {
             float4* c = ck + (size_t)stored * (TW * TH);
 #pragma unroll
             for (int h = 0; h < PX; ++h)
               c[h * kHalf] = make_float4(L::get(T, h), L::get(S0, h), L::get(S1, h), L::get(S2, h));
             S0 = S1 = S2 = L::all(0.f);
             ++stored;
+            seg_end = stored + 1 < a.b.seg_k ? s0 + segs.begin(stored + 1) : 0u;  // the last one is open-ended
           }
         }
       }
@@ -634,6 +653,17 @@ __global__ void __launch_bounds__(SPLIT ? 64 : TW * TH / 2, SPLIT ? 8 : CKPT ? 4
       if (__syncthreads_and(saturated())) break;
     }
     if constexpr (CKPT) {
+      // A split tile's CTA may stop, saturated, before the tile does: its pixels'
+      // last entries then lie in a segment that other CTAs see the end of, and the
+      // state there is the present one.
+      if (SPLIT && stored + 1 < a.b.seg_k) {
+        float4* c = ck + (size_t)stored * (TW * TH);
+#pragma unroll
+        for (int h = 0; h < PX; ++h)
+          c[h * kHalf] = make_float4(L::get(T, h), L::get(S0, h), L::get(S1, h), L::get(S2, h));
+        S0 = S1 = S2 = L::all(0.f);
+        ++stored;
+      }
       // Each thread turns its own checkpoints' colours into the sum over the
       // later segments, from the last one forward.
       for (int k = (int)stored - 1; k >= 0; --k) {
@@ -687,22 +717,21 @@ __global__ void __launch_bounds__(SPLIT ? 64 : TW * TH / 2, SPLIT ? 8 : CKPT ? 4
     }
     if (!SPLIT || top != 0xffffffffu) {
       const uint32_t cost = top > s0 ? top - s0 : 0u;
-      bool split = false;
-      if (!CKPT && TW == 16 && TH == 16 && a.long_tiles && cost > kLongTile) {
-        // Room for kLongTiles of them; tile_sync is free in a launch without checkpoints.
-        if (threadIdx.x == 0 && (s_item = atomicAdd(a.b.tile_sync, 1u)) < kLongTiles) {
-          const uint32_t c = cost_bucket(cost / 2);
+      for (uint32_t g = threadIdx.x; g < (CKPT ? a.b.seg_k : 1u); g += NT) {  // the tile's backward items
+        const uint32_t lo = CKPT ? segs.begin(g) : 0u;
+        if (g > 0 && lo >= cost) break;
+        const uint32_t n = (CKPT && g + 1 < a.b.seg_k ? min(segs.begin(g + 1), cost) : cost) - lo;
+        const uint32_t work = item * a.b.seg_k + g;
+        if (TW == 16 && TH == 16 && a.long_tiles && n > kLongTile && atomicAdd(a.b.long_count, 1u) < kLongTiles) {
+          // A long walk: an item per 8x8 block.
+          const uint32_t c = cost_bucket(n / 2);
           const uint32_t at = atomicAdd(a.b.sched_lcount + c, 4u);
           for (uint32_t q = 0; q < 4; ++q)
-            a.b.sched_lists[(size_t)c * a.b.sched_items_cap + at + q] = item | (q + 1) << kBlockShift;
+            a.b.sched_lists[(size_t)c * a.b.sched_items_cap + at + q] = work | (q + 1) << kBlockShift;
+        } else {
+          const uint32_t c = cost_bucket(n);
+          a.b.sched_lists[(size_t)c * a.b.sched_items_cap + atomicAdd(a.b.sched_lcount + c, 1u)] = work;
         }
-        __syncthreads();
-        split = s_item < kLongTiles;
-      }
-      const uint32_t nseg = split ? 0u : CKPT ? min(a.b.seg_k, max((cost + seg_len - 1u) / seg_len, 1u)) : 1u;
-      for (uint32_t g = threadIdx.x; g < nseg; g += NT) {  // the tile's backward items, one per segment
-        const uint32_t c = cost_bucket(g + 1 < nseg ? seg_len : cost - g * seg_len);
-        a.b.sched_lists[(size_t)c * a.b.sched_items_cap + atomicAdd(a.b.sched_lcount + c, 1u)] = item * a.b.seg_k + g;
       }
     }
     __syncthreads();
@@ -1219,9 +1248,10 @@ __global__ void __launch_bounds__(32, kTileBwdBlocks) raster_bwd_tile_kernel(Ras
   for (uint32_t round = 0;; ++round) {
     const uint32_t work = next_item<SEG>(a, round, &s_item, &s_lists);
     if (work == kNoItem) break;
-    const uint32_t item = SEG ? work / a.b.seg_k : work & ((1u << kBlockShift) - 1u), seg = SEG ? work % a.b.seg_k : 0u;
-    // The 8x8 blocks this item takes: all, or one of a long list.
-    const uint32_t blocks = SEG || work < (1u << kBlockShift) ? 0xfu : 1u << ((work >> kBlockShift) - 1u);
+    // The 8x8 blocks this item takes: all, or one of a long walk.
+    const uint32_t blocks = work < (1u << kBlockShift) ? 0xfu : 1u << ((work >> kBlockShift) - 1u);
+    const uint32_t id = work & ((1u << kBlockShift) - 1u);
+    const uint32_t item = SEG ? id / a.b.seg_k : id, seg = SEG ? id % a.b.seg_k : 0u;
     const uint32_t v = find_view(a.vs, item);
     const ViewDesc& vd = a.vs.views[v];
     const uint32_t t = item - vd.tile_base;
@@ -1234,7 +1264,7 @@ __global__ void __launch_bounds__(32, kTileBwdBlocks) raster_bwd_tile_kernel(Ras
                           -((float)(py0 + 12) + 0.5f)};
     const uint32_t* ranges = slice(a.b.ranges, 2 * a.b.Tcap, v);
     const uint32_t s0 = ranges[2 * t];
-    const uint32_t seg_len = SEG ? segment_len(ranges[2 * t + 1] - s0, a.b.seg_k) : 0u;
+    const Segments segs = segments_of(ranges[2 * t + 1] - s0, SEG ? a.b.seg_k : 1u);
     const uint32_t* vals = isect_index_src(a.b, v);
     const uint32_t vmask = isect_index_mask(a.b);
     const float4* rec = slice(a.b.rec, a.b.Vcap * 3, v);
@@ -1255,12 +1285,13 @@ __global__ void __launch_bounds__(32, kTileBwdBlocks) raster_bwd_tile_kernel(Ras
     // This segment's entries [lo, hi); the last segment ends at the tile's
     // last contributor and starts from the pixels' final state, the others
     // from their checkpoint.
-    const uint32_t lo = SEG ? s0 + seg * seg_len : s0;
+    const uint32_t lo = SEG ? s0 + segs.begin(seg) : s0;
     if (SEG && seg > 0 && lo >= smax) continue;  // grid schedule: past the tile's segments
-    const bool final_seg = !SEG || seg + 1 == a.b.seg_k || smax <= lo + seg_len;
-    const uint32_t hi = final_seg ? smax : lo + seg_len;
+    const uint32_t end = SEG ? s0 + segs.begin(seg + 1) : 0u;
+    const bool final_seg = !SEG || seg + 1 == a.b.seg_k || smax <= end;
+    const uint32_t hi = final_seg ? smax : end;
     if (!final_seg) {
-      const float4* ck = a.b.ckpt + (size_t)work * 256 + lane;
+      const float4* ck = a.b.ckpt + (size_t)id * 256 + lane;
   #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const float4 u = ck[q * 32], w = ck[128 + q * 32];

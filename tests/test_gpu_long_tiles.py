@@ -14,12 +14,12 @@ pytestmark = pytest.mark.gpu
 W, H = 1056, 1040  # 66 x 65 tiles
 
 
-def _scene(n):
-    """n small faint Gaussians inside tile (20, 30), 200 larger ones anywhere."""
+def _scene(n, W=W, H=H, tx=20, ty=30):
+    """n small faint Gaussians inside tile (tx, ty), 200 larger ones anywhere."""
     rng = np.random.default_rng(n)
     f, z = 1000.0, 2.0 + 2.0 * rng.random(n + 200)
-    u = np.concatenate([20 * 16 + 1 + 14 * rng.random(n), W * rng.random(200)])
-    v = np.concatenate([30 * 16 + 1 + 14 * rng.random(n), H * rng.random(200)])
+    u = np.concatenate([tx * 16 + 1 + 14 * rng.random(n), W * rng.random(200)])
+    v = np.concatenate([ty * 16 + 1 + 14 * rng.random(n), H * rng.random(200)])
     tr = np.zeros((n + 200, 10), np.float32)
     tr[:, 0], tr[:, 1], tr[:, 2] = (u - W / 2) * z / f, (v - H / 2) * z / f, z
     tr[:, 3:7] = rng.standard_normal((n + 200, 4))
@@ -54,3 +54,27 @@ def test_long_tile_parity(gsr_ctx_factory, n, deterministic):
     for k, a in res[0].items():
         assert_grad_parity(a, b32[k], b64[k], what=f"{n} {k}")
         np.testing.assert_array_equal(a, res[-1][k])
+
+
+@pytest.mark.parametrize("deterministic", [False, True])
+@pytest.mark.parametrize("w,h,n", [(64, 48, 4000), (64, 48, 9000), (400, 300, 6000), (1024, 1000, 3000), (1024, 1000, 12000)])
+def test_long_list_of_few_tiles_parity(gsr_ctx_factory, w, h, n, deterministic):
+    """Launches of at most 4096 tiles, whose lists are cut into segments that grow
+    along the list: one list far longer than the short segments cover, with 64,
+    33 and 4 segments a tile, and a last segment of more than 4096 entries."""
+    import torch
+
+    from rustscan_b200 import host_splats_to_device
+
+    sc = _scene(n, w, h, w // 32, h // 32)
+    ctx = gsr_ctx_factory(max_splats=sc.n, max_pixels=w * h, deterministic=deterministic)
+    splats = host_splats_to_device(sc)
+    up = S.upstream_grad(h, w, seed=n)
+    _, g = run_gpu_forward(ctx, splats, sc.cameras)
+    gr = ctx.render_backward(splats, torch.as_tensor(up.reshape(-1), device="cuda"))
+    torch.cuda.synchronize()
+    o = oracle_forward(sc, sc.cameras[0])
+    assert_forward_parity(g[0], o)
+    b32, b64 = o.backward(up, mode=0), oracle_forward(sc, sc.cameras[0], f64=True).backward(up, mode=0)
+    for k in ("v_transforms", "v_sh", "v_raw_opacity"):
+        assert_grad_parity(gr[k].cpu().numpy(), b32[k], b64[k], what=f"{w}x{h} {n} {k}")
