@@ -29,7 +29,7 @@ UNIT = "ms/view"
 WORKLOAD = "batched training step: 1,000,000 Gaussians, SH degree 3, 8 views of 1280x720 per step"
 # ncu smsp__inst_executed.sum of the raster kernels on one 1280x720 view of
 # this workload (6,273,269 intersections), per intersection
-# (profiles/raster_c3_1view_issue.md).
+# (profiles/kernels_c3_2views.md).
 WARP_INST_PER_ISECT = {"raster_bwd": 153.95e6 / 6273269, "raster_fwd": 134.88e6 / 6273269}
 
 
@@ -660,7 +660,8 @@ def main():
         "raster_bwd": sum(40 * I[v] + 32 * P + 56 * V[v] for v in range(nv)),
         "tile_sort": sum(16 * I[v] for v in range(nv)),  # two passes over packed 4-byte keys, read + write
         "project": 44 * args.n + sum((12 + 48 + 192) * V[v] for v in range(nv)),
-        "adam": 28 * (10 + 48 + 1) * args.n + 8 * 10 * args.n,
+        # Parameters and moments read and written, the views' gradient sums read.
+        "project_bwd": 24 * (10 + 48 + 1) * args.n + sum(48 * V[v] for v in range(nv)),
     }
     dom = max((k for k in algo), key=lambda k: stages.get(k, 0.0))
     achieved = algo[dom] / (stages[dom] * 1e-3) / 1e9
@@ -673,8 +674,6 @@ def main():
                      "tile_sort": (30.3e6 + 0.4e6 + 30.4e6 + 0.6e6) / 6273269}
     if dom in traffic_coeff:
         traffic = traffic_coeff[dom] * sum(I)
-    elif dom == "adam":
-        traffic = (160.0e6 + 63.1e6 + 768.0e6 + 520.4e6 + 16.0e6) * args.n / 1_000_000
     else:
         traffic = None
     roofline = {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": hbm, "unit": "GB/s",
