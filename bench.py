@@ -27,10 +27,10 @@ sys.path.insert(0, ROOT)
 METRIC = "fwd+bwd ms/view (1M Gaussians, 1280x720) batched vs plain; grad rel err"
 UNIT = "ms/view"
 WORKLOAD = "batched training step: 1,000,000 Gaussians, SH degree 3, 8 views of 1280x720 per step"
-# ncu smsp__inst_executed.sum of the raster kernels on one 1280x720 view of
-# this workload (6,273,269 intersections), per intersection
+# ncu smsp__inst_executed.sum of the raster kernels on the first two 1280x720
+# views of this workload (12,531,620 intersections), per intersection
 # (profiles/kernels_c3_2views.md).
-WARP_INST_PER_ISECT = {"raster_bwd": 153.95e6 / 6273269, "raster_fwd": 134.88e6 / 6273269}
+WARP_INST_PER_ISECT = {"raster_bwd": 316.1e6 / 12531620, "raster_fwd": 177.5e6 / 12531620}
 
 
 def parse():
@@ -666,12 +666,11 @@ def main():
     dom = max((k for k in algo), key=lambda k: stages.get(k, 0.0))
     achieved = algo[dom] / (stages[dom] * 1e-3) / 1e9
     # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) from one ncu
-    # capture of a single 1280x720 view of this workload (6,273,269
+    # capture of the first two 1280x720 views of this workload (12,531,620
     # intersections), scaled to the launch by its intersections (the raster
-    # and tile-sort traffic grows with them) or, for Adam, taken as is (it
-    # sweeps the N parameters once per step).
-    traffic_coeff = {"raster_bwd": (37.736e6 + 0.016e6) / 6273269, "raster_fwd": (14.121e6 + 0.219e6) / 6273269,
-                     "tile_sort": (30.3e6 + 0.4e6 + 30.4e6 + 0.6e6) / 6273269}
+    # and tile-sort traffic grows with them).
+    traffic_coeff = {"raster_bwd": (78.6e6 + 2.5e6) / 12531620, "raster_fwd": (30.4e6 + 13.0e6) / 12531620,
+                     "tile_sort": (59.3e6 + 8.1e6 + 52.4e6 + 9.9e6) / 12531620}
     if dom in traffic_coeff:
         traffic = traffic_coeff[dom] * sum(I)
     else:
@@ -684,7 +683,7 @@ def main():
     # issue roofline is the SMs' warp-instruction issue rate (4 schedulers
     # per SM, one warp instruction each per clock) at the SM clock measured
     # during the timed region. The warp instructions per launch come from
-    # one ncu capture of a single 1280x720 view (smsp__inst_executed.sum),
+    # one ncu capture of two 1280x720 views (smsp__inst_executed.sum),
     # scaled to the launch by its intersections.
     inst_per_isect = {"raster_bwd": WARP_INST_PER_ISECT["raster_bwd"], "raster_fwd": WARP_INST_PER_ISECT["raster_fwd"]}
     sm_mhz = clk.summary().get("sm_mhz") or 1965.0
@@ -696,8 +695,8 @@ def main():
                              "peak": peak_issue / 1e9, "unit": "G warp-instructions/s",
                              "frac": winst / (stages[dom] * 1e-3) / peak_issue, "warp_instructions": winst,
                              "sm_mhz": sm_mhz, "sms": n_sm,
-                             "source": "warp instructions per intersection from ncu smsp__inst_executed.sum on one "
-                                       "view, times this launch's intersections"}
+                             "source": "warp instructions per intersection from ncu smsp__inst_executed.sum on two "
+                                       "views, times this launch's intersections"}
 
     # ---- the same batched step with BF16 SH storage ---------------------------
     bf16_ms = None
