@@ -378,6 +378,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) cluster_sort_kernel(Cluste
   extern __shared__ uint4 smem_cs[];
   ClusterSortSmem<C, IT>& S = *reinterpret_cast<ClusterSortSmem<C, IT>*>(smem_cs);
   cg::cluster_group cluster = cg::this_cluster();
+  cluster.barrier_arrive();  // this CTA has started; the loads below hide the wait for the others
   const uint32_t rank = cluster.block_rank(), v = blockIdx.y;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t V = a.vcount[v * 4 + 0];
@@ -413,6 +414,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) cluster_sort_kernel(Cluste
   __syncthreads();
   lo = __reduce_min_sync(0xffffffffu, S.red[0][lane]);
   hi = __reduce_max_sync(0xffffffffu, S.red[1][lane]);
+  cluster.barrier_wait();  // every CTA has started: its shared memory may be written
   if (tid < (uint32_t)C) *cluster.map_shared_rank(&S.range[rank], tid) = make_uint2(lo, hi);
   cluster.sync();
 #pragma unroll
