@@ -142,9 +142,10 @@ __device__ __forceinline__ ViewAdjoint view_adjoint(const BwdView& w, V3<float> 
   // Compensation sqrt(det / det of the blurred), and the conic (inverse2x2_packed).
   const float d00 = s00 + blur, d11 = s11 + blur;
   const float det_raw = fmaxf(s00 * s11 - s01 * s01, 0.f), det_blur = d00 * d11 - s01 * s01;
-  const float det_end = fmaxf(det_blur, 1e-12f), rend = rcp_newton(det_end);
-  const float root = det_raw > 0.f ? rsqrt_newton(det_raw * det_end) : 0.f;  // compensation / det_raw
-  float fc = det_raw * root;
+  const float det_end = fmaxf(det_blur, 1e-12f);
+  const float ratio = det_raw / det_end;  // a product of both overflows from a projection of 65,500 pixels on
+  const float comp = sqrtf(ratio);
+  float fc = comp;
   const float i00 = d00 + 1e-6f, i11 = d11 + 1e-6f, det = i00 * i11 - s01 * s01;
   const float inv = det > 1e-10f ? rcp_newton(det) : 0.f;
   V3<float> ci{i11 * inv, -s01 * inv, i00 * inv};
@@ -158,17 +159,17 @@ __device__ __forceinline__ ViewAdjoint view_adjoint(const BwdView& w, V3<float> 
   }
   o.v_raw_opac = fc * q2.x * opac * (1.f - opac);
   // G: gradient of the 2D covariance, -C V C, and through the compensation
-  // (compensate_vjp).
+  // (compensate_vjp, whose factor 1 / det_end is ratio / det_raw).
   const float v0 = q0.z, vh = 0.5f * q0.w, v2 = q1.x;
   const float t00 = ci.x * v0 + ci.y * vh, t01 = ci.x * vh + ci.y * v2;
   const float t10 = ci.y * v0 + ci.z * vh, t11 = ci.y * vh + ci.z * v2;
   float g00 = -(t00 * ci.x + t01 * ci.y), g01 = -(t00 * ci.y + t01 * ci.z), g11 = -(t10 * ci.y + t11 * ci.z);
   if (exact) {
-    const float h = 0.5f * q2.x * opac, k0 = h * root;
-    const float k1 = det_blur > 1e-12f ? h * det_raw * root * rend : 0.f;
-    g00 += k0 * s11 - k1 * d11;
-    g01 += (k1 - k0) * s01;
-    g11 += k0 * s00 - k1 * d00;
+    const float k = det_raw > 0.f ? (0.5f * q2.x * opac * comp) / det_raw : 0.f;
+    const float rk = det_blur > 1e-12f ? ratio : 0.f;
+    g00 += k * (s11 - rk * d11);
+    g01 += k * (rk - 1.f) * s01;
+    g11 += k * (s00 - rk * d00);
   }
   // H = G J: rows (g00 jx, g01 jy, e0) and (g01 jx, g11 jy, e1).
   const float e0 = g00 * a + g01 * b, e1 = g01 * a + g11 * b;
@@ -292,8 +293,8 @@ __device__ __forceinline__ void stage_sh_rows(const __nv_bfloat16* src, uint32_t
 // of the DRAM rate and of the issue slots each. It replaces a pass per (view,
 // Gaussian) that wrote 96-byte adjoint records, a pass that summed them and, in
 // a training step, the Adam passes that read the gradient back: 8 views of 1M
-// Gaussians 0.817 -> 0.573 ms, 16 uneven views of 2M (BF16 SH) 2.77 -> 1.63, one
-// view of 3M (BF16, gradients out) 0.548 -> 0.386.
+// Gaussians 0.817 -> 0.624 ms, 16 uneven views of 2M (BF16 SH) 2.77 -> 1.80, one
+// view of 3M (BF16, gradients out) 0.548 -> 0.402.
 // Degree 4 runs three blocks per SM at 168 registers with a few spills: 300k
 // Gaussians at 640x480, gradient and Adam, 263 us with two blocks, 223 so (the
 // separate passes took 223), 600k in 5 views 615 and 534 (603), 659k in 2 600 and
