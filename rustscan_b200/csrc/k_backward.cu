@@ -88,19 +88,6 @@ __device__ __forceinline__ void load_view(const ViewDesc& d, BwdView& o) {
   o.ylo = (-0.15f * (float)d.h - d.cy) / d.fy;
 }
 
-// 1 / x and 1 / sqrt(x) from the hardware's estimates and one Newton step each
-// (x + x (1 - a x) and y + y (1/2 - a y^2 / 2)), about one unit in the last
-// place, for normal a > 0.
-__device__ __forceinline__ float rcp_newton(float a) {
-  float x;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(x) : "f"(a));
-  return fmaf(x, fmaf(-a, x, 1.f), x);
-}
-__device__ __forceinline__ float rsqrt_newton(float a) {
-  const float y = rsqrtf(a);
-  return fmaf(y, fmaf(-0.5f * a * y, y, 0.5f), y);
-}
-
 // The projection adjoint of one view (project_backward without the SH terms):
 // adds into the gradients of the mean and, as the symmetric matrix (xx, xy, xz,
 // yy, yz, zz), of the 3D covariance, returns the opacity logit's. Written out
@@ -131,7 +118,7 @@ __device__ __forceinline__ ViewAdjoint view_adjoint(const BwdView& w, V3<float> 
   auto m = [&](int i, int j) { return A[i][0] * R[j] + A[i][1] * R[3 + j] + A[i][2] * R[6 + j]; };
   const float M00 = m(0, 0), M01 = m(0, 1), M02 = m(0, 2), M11 = m(1, 1), M12 = m(1, 2), M22 = m(2, 2);
   // The Jacobian's rows (jx, 0, a) and (0, jy, b).
-  const float rz = rcp_newton(fmaxf(z, 0.01f));
+  const float rz = 1.f / fmaxf(z, 0.01f);
   const float xr = x * rz, yr = y * rz;
   const float uc = fminf(fmaxf(xr, w.xlo), w.xhi), vc = fminf(fmaxf(yr, w.ylo), w.yhi);
   const float jx = w.fx * rz, jy = w.fy * rz, a = -jx * uc, b = -jy * vc;
@@ -147,7 +134,7 @@ __device__ __forceinline__ ViewAdjoint view_adjoint(const BwdView& w, V3<float> 
   const float comp = sqrtf(ratio);
   float fc = comp;
   const float i00 = d00 + 1e-6f, i11 = d11 + 1e-6f, det = i00 * i11 - s01 * s01;
-  const float inv = det > 1e-10f ? rcp_newton(det) : 0.f;
+  const float inv = det > 1e-10f ? 1.f / det : 0.f;
   V3<float> ci{i11 * inv, -s01 * inv, i00 * inv};
   if (hp) {
     M2<float> cov;
@@ -293,8 +280,10 @@ __device__ __forceinline__ void stage_sh_rows(const __nv_bfloat16* src, uint32_t
 // of the DRAM rate and of the issue slots each. It replaces a pass per (view,
 // Gaussian) that wrote 96-byte adjoint records, a pass that summed them and, in
 // a training step, the Adam passes that read the gradient back: 8 views of 1M
-// Gaussians 0.817 -> 0.624 ms, 16 uneven views of 2M (BF16 SH) 2.77 -> 1.80, one
-// view of 3M (BF16, gradients out) 0.548 -> 0.402.
+// Gaussians 0.817 -> 0.625 ms, 16 uneven views of 2M (BF16 SH) 2.77 -> 1.81, one
+// view of 3M (BF16, gradients out) 0.548 -> 0.406. Correctly rounded divisions
+// and roots are 6% to 10% of that: with estimates and a Newton step each it took
+// 0.573, 1.63 and 0.386.
 // Degree 4 runs three blocks per SM at 168 registers with a few spills: 300k
 // Gaussians at 640x480, gradient and Adam, 263 us with two blocks, 223 so (the
 // separate passes took 223), 600k in 5 views 615 and 534 (603), 659k in 2 600 and
@@ -379,7 +368,7 @@ __global__ void __launch_bounds__(kGT, DEG >= 4 ? 3 : 4) gather_kernel(GatherArg
         // (sh_viewdir_vjp).
         V3<float> dir{mean.x - w.campos[0], mean.y - w.campos[1], mean.z - w.campos[2]};
         const float n2 = dir.x * dir.x + dir.y * dir.y + dir.z * dir.z;
-        const float rn = rsqrt_newton(fmaxf(n2, 1e-12f));
+        const float rn = 1.f / sqrtf(fmaxf(n2, 1e-12f));
         dir = V3<float>{dir.x * rn, dir.y * rn, dir.z * rn};
         const float rgb[3] = {q1.y, q1.z, q1.w};
         if (dir_term) {
