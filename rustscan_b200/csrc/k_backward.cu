@@ -280,14 +280,14 @@ __device__ __forceinline__ void stage_sh_rows(const __nv_bfloat16* src, uint32_t
 // of the DRAM rate and of the issue slots each. It replaces a pass per (view,
 // Gaussian) that wrote 96-byte adjoint records, a pass that summed them and, in
 // a training step, the Adam passes that read the gradient back: 8 views of 1M
-// Gaussians 0.817 -> 0.625 ms, 16 uneven views of 2M (BF16 SH) 2.77 -> 1.81, one
+// Gaussians 0.817 -> 0.626 ms, 16 uneven views of 2M (BF16 SH) 2.77 -> 1.82, one
 // view of 3M (BF16, gradients out) 0.548 -> 0.406. Correctly rounded divisions
 // and roots are 6% to 10% of that: with estimates and a Newton step each it took
 // 0.573, 1.63 and 0.386.
-// Degree 4 runs three blocks per SM at 168 registers with a few spills: 300k
-// Gaussians at 640x480, gradient and Adam, 263 us with two blocks, 223 so (the
-// separate passes took 223), 600k in 5 views 615 and 534 (603), 659k in 2 600 and
-// 492 (522).
+// Degree 4 runs three blocks per SM at 168 registers with a few spills: gradient
+// and Adam of 300k Gaussians at 640x480 225 us (the separate passes 220), 600k in
+// 5 views 560 (604), 659k in 2 501 (514); with two blocks 263, 615 and 600, when
+// three took 223, 534 and 492.
 template <class SHT, int DEG>
 __global__ void __launch_bounds__(kGT, DEG >= 4 ? 3 : 4) gather_kernel(GatherArgs a) {
   constexpr int K = (DEG + 1) * (DEG + 1);
@@ -408,7 +408,9 @@ __global__ void __launch_bounds__(kGT, DEG >= 4 ? 3 : 4) gather_kernel(GatherArg
         if (a.acc) {
           // Densification quantities of this view (engine/trainer.rs:660-727),
           // one view at a time, in view order, as a per-view accumulation does.
-          S.acc[0][r] += (fabsf(o.v_mean.x) + fabsf(o.v_mean.y) + fabsf(o.v_mean.z)) * (1.0f / 3.0f);
+          // A third, correctly rounded: a quotient by 3 lies too far from the middle
+          // of two floats for the product in 64 bits to round otherwise.
+          S.acc[0][r] += (float)((double)(fabsf(o.v_mean.x) + fabsf(o.v_mean.y) + fabsf(o.v_mean.z)) * (1.0 / 3.0));
           S.acc[1][r] += sqrtf(st[0] * st[0] + st[1] * st[1]);
           S.acc[2][r] += sqrtf(st[2] * st[2] + st[3] * st[3]);
           S.acc[3][r] += st[4];
