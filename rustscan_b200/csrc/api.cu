@@ -161,6 +161,7 @@ gsr_status allocate(gsr_ctx* c) {
             dalloc(c, &b.sched_lcount, kSchedWords) && dalloc(c, &b.sched_ticket, 1);
   b.tile_sync = b.sched_lcount + 32;
   b.long_count = b.tile_sync + 2 * kFwdSplitTiles;
+  b.inf_colour = b.long_count + 1;
   // Backward work items: the tiles, or the segments of a launch of few tiles.
   b.sched_items_cap = std::max<uint64_t>(nv * T, kSegItems) + 3 * kLongTiles;
   ok = ok && dalloc(c, &b.sched_lists, 32 * b.sched_items_cap);

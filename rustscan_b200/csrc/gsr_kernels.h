@@ -48,6 +48,7 @@ struct FwdBufs {
   uint32_t* sched_lcount;  // [32] items in each of those lists (appended by the forward)
   uint32_t* tile_sync;     // [kFwdSplitTiles][2] split forward, after sched_lcount: largest last contributor, CTAs done
   uint32_t* long_count;    // items of long walks listed block by block
+  uint32_t* inf_colour;    // set by the projection if a record holds an infinite colour
   uint32_t* sched_ticket;  // [1] next ticket a persistent raster CTA takes
   uint64_t sched_items_cap;
   float4* ckpt;            // [kSegItems][256] per (tile, segment) and pixel: transmittance after it, colour behind it
@@ -98,8 +99,8 @@ constexpr uint32_t kFwdSplitTiles = 1024, kFwdSplitSplats = 32;
 // 2.92 both, where the blocks' extra reductions cost 2% from 1024 entries and 0.6%
 // from 2048; from 8192 on the second case takes 1.29.
 constexpr uint32_t kLongTile = 4096, kLongTiles = 4096;
-// Words of sched_lcount with tile_sync and long_count behind it.
-constexpr uint32_t kSchedWords = 32 + 2 * kFwdSplitTiles + 1;
+// Words of sched_lcount with tile_sync, long_count and inf_colour behind it.
+constexpr uint32_t kSchedWords = 32 + 2 * kFwdSplitTiles + 2;
 
 // Bits of ViewSet::persistent (otherwise one CTA per work item).
 constexpr int kPersistFwd = 1, kPersistBwd = 2;
@@ -137,8 +138,8 @@ constexpr uint32_t kProjBlock = 256;
 
 // ---- launchers (return cudaGetLastError()) ----
 // Projects, compacts and colours all views; also writes the view descriptors
-// (host_views) to dev_views and clears tile_hist, sched_lcount with tile_sync,
-// and visible_c.
+// (host_views) to dev_views and clears tile_hist, visible_c, and sched_lcount
+// with what lies behind it (see kSchedWords).
 cudaError_t launch_project(const SplatsDev& sp, const ViewSet& vs, const ViewDesc* host_views, ViewDesc* dev_views,
                            float cov_blur, int fp64_conic, FwdBufs& b, cudaStream_t st);
 

@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kProjThreads)
   if (part == 0)
     for (uint32_t v = threadIdx.x; v < nv; v += kProjThreads) a.views[v] = blk.v[v];
   // Counters of the later stages: tile counts, and the cost lists' counts with
-  // the split tiles' meeting places behind them.
+  // the split tiles' meeting places and the flag of pass 3 behind them.
   for (uint32_t v = 0; v < nv; ++v)
     for (uint32_t t = g0 + threadIdx.x; t < blk.v[v].tiles_x * blk.v[v].tiles_y; t += a.parts * kProjThreads)
       slice(a.b.tile_hist, a.b.Tcap, v)[t] = 0u;
@@ -296,6 +296,7 @@ __global__ void __launch_bounds__(kProjThreads)
       r[1] = make_float4(p.conic.z, p.opacity, rgb.x, rgb.y);
       r[2] = make_float4(rgb.z, p.thr, __uint_as_float(p.box.x0 | (p.box.x1 << 16)),
                          __uint_as_float(p.box.y0 | (p.box.y1 << 16)));
+      if (fmaxf(fmaxf(rgb.x, rgb.y), rgb.z) == INFINITY) *a.b.inf_colour = 1u;
       slice(a.b.gid_of_c, a.b.Vcap, v)[c] = g;
       slice(a.b.depth_key, a.b.Vcap, v)[c] = __float_as_uint(p.depth);
       slice(a.b.visible_c, a.b.Vcap, v)[c] = 0;

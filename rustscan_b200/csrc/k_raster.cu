@@ -344,6 +344,7 @@ template <> struct Lane<2> {
   __device__ static V all(float x) { return make_float2(x, x); }
   __device__ static V of(float2 twice) { return twice; }
   __device__ static V make(const float (&x)[2]) { return make_float2(x[0], x[1]); }
+  __device__ static V pick(const bool (&c)[2], V a, V b) { return make_float2(c[0] ? a.x : b.x, c[1] ? a.y : b.y); }
   __device__ static float get(V v, int h) { return h ? v.y : v.x; }
 };
 template <> struct Lane<1> {
@@ -351,6 +352,7 @@ template <> struct Lane<1> {
   __device__ static V all(float x) { return x; }
   __device__ static V of(float2 twice) { return twice.x; }
   __device__ static V make(const float (&x)[1]) { return x[0]; }
+  __device__ static V pick(const bool (&c)[1], V a, V b) { return c[0] ? a : b; }
   __device__ static float get(V v, int) { return v; }
 };
 
@@ -392,6 +394,14 @@ struct __align__(16) FwdEntry {
 // Entries a warp evaluates together. Two cost nothing on large launches but
 // 2% on a launch of 300 tiles, where few warps hide each other's latency.
 constexpr int kFwdUnroll = 4;
+template <int BATCH, int NW> struct FwdSmem {
+  FwdEntry e[BATCH + 1];  // the last one is never taken: it pads the lists
+  uint8_t mask[BATCH];
+  alignas(8) uint16_t list[NW][BATCH + kFwdUnroll];  // byte offsets into e
+  uint32_t item;
+  uint32_t work;  // the item's largest last contributor
+  uint32_t top;   // the tile's, in the last of a split tile's CTAs
+};
 // Resident threads per SM the register bound allows (768: 80 registers): 8
 // views of 1280x720 blend in 0.832 ms, in 0.844 at 640 and 0.830 with more
 // spills at 896.
@@ -404,8 +414,8 @@ constexpr int kFwdThreadsPerSm = 768;
 // independent of the pixel state and run as one straight-line block, so their
 // latencies overlap; the four blends then follow in order. No branch depends
 // on a pixel: a pixel that does not take an entry blends with alpha 0, which
-// leaves its colour and transmittance bit for bit unchanged, and a saturated
-// pixel (transmittance below 1e-4) takes nothing. What bounds it is
+// leaves its transmittance and, where all colours are finite, its colour bit for
+// bit unchanged, and a saturated pixel (transmittance below 1e-4) takes nothing. What bounds it is
 // instruction issue and, on launches of few tiles, the latency of the
 // longest tile. Against a walk of two entries with a vote and
 // a branch each, over blocks culled by the footprint's bounding box: 8 views
@@ -423,32 +433,36 @@ constexpr int kFwdThreadsPerSm = 768;
 // one pixel per lane, each walking the entries that reach its 8x4 strip (see
 // kFwdSplitTiles). The four CTAs of a tile set their hit bits one by one, and
 // the last of them lists the tile for the backward.
-template <int TW, int TH, int BATCH, bool CKPT, bool SPLIT>
-__global__ void __launch_bounds__(SPLIT ? 64 : TW * TH / 2, SPLIT ? 8 : CKPT ? 4 : kFwdThreadsPerSm / (TW * TH / 2))
-    raster_fwd_kernel(RasterArgs a) {
+// FINITE: no colour is infinite. 0 times infinity is not 0, so otherwise a pixel
+// that does not take an entry keeps its sums by selection. That costs a split
+// tile's lanes, of one pixel each, up to 2 us (300 tiles over 74k Gaussians 80.5 ->
+// 82.4), but 14% with two pixels and checkpoints (1200 tiles over 200k 93 -> 106);
+// so the launches that are not split take it only if the projection reports an
+// infinite colour. The report's load takes 0.6% of a large launch (8 views of
+// 1280x720 0.822 -> 0.827 ms).
+template <int TW, int TH, int BATCH, bool CKPT, bool SPLIT, bool FINITE>
+__device__ __forceinline__ void blend_items(const RasterArgs& a, FwdSmem<BATCH, SPLIT ? 2 : TW * TH / 64>& S) {
   constexpr int PX = SPLIT ? 1 : 2;  // pixels per lane
   using L = Lane<PX>;
   using V = typename L::V;
   constexpr int NT = SPLIT ? 64 : TW * TH / 2;
   constexpr int NW = NT / 32;
-  constexpr int S = 2 / PX;                   // warps per 8x8 block
+  constexpr int WB = 2 / PX;                  // warps per 8x8 block
   constexpr int BW = SPLIT ? 8 : TW;          // width of the CTA's pixel area
   constexpr int kSI = (BATCH + NT - 1) / NT;  // entries a thread stages per batch
-  static_assert(NW / S <= 4 && TW % 8 == 0 && TH % 8 == 0, "hit bits of at most four 8x8 blocks");
-  __shared__ FwdEntry s_e[BATCH + 1];  // the last one is never taken: it pads the lists
-  __shared__ uint8_t s_mask[BATCH];
-  __shared__ __align__(8) uint16_t s_list[NW][BATCH + kFwdUnroll];  // byte offsets into s_e
-  __shared__ uint32_t s_item;
-  __shared__ uint32_t s_work;
+  static_assert(NW / WB <= 4 && TW % 8 == 0 && TH % 8 == 0, "hit bits of at most four 8x8 blocks");
+  auto& s_e = S.e;
+  auto& s_mask = S.mask;
+  uint32_t& s_work = S.work;
   if (threadIdx.x == 0) {
     s_work = 0u;
     s_e[BATCH] = FwdEntry{};  // sigma 0, opacity 0: alpha 0
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int half = warp % S;  // SPLIT: the block's rows y + 4 half
-  uint16_t* list = s_list[warp];
+  const int half = warp % WB;  // SPLIT: the block's rows y + 4 half
+  uint16_t* list = S.list[warp];
   for (uint32_t round = 0;; ++round) {
-    const uint32_t work = next_item<SPLIT ? 4 : 1>(a, round, &s_item);
+    const uint32_t work = next_item<SPLIT ? 4 : 1>(a, round, &S.item);
     if (work == kNoItem) break;
     const uint32_t item = SPLIT ? work / 4 : work;
     const int block = SPLIT ? (int)(work % 4) : warp;  // 8x8 block of the tile
@@ -522,7 +536,7 @@ __global__ void __launch_bounds__(SPLIT ? 64 : TW * TH / 2, SPLIT ? 8 : CKPT ? 4
       E.last = i + 1;
       *reinterpret_cast<uint32_t*>(E.hit) = 0u;
       E.cidx = r.c;
-      s_mask[j] = (uint8_t)reached_blocks<BW, NW, 8 / S>(r.r0.x, r.r0.y, r.r0.z, r.r0.w, r.r1.x, cut, tx0, ty0);
+      s_mask[j] = (uint8_t)reached_blocks<BW, NW, 8 / WB>(r.r0.x, r.r0.y, r.r0.z, r.r0.w, r.r1.x, cut, tx0, ty0);
     };
     Raw next[CKPT ? kSI : 1];  // CKPT: this thread's entries of the next batch
     auto fetch = [&](uint32_t b0) {
@@ -592,13 +606,17 @@ __global__ void __launch_bounds__(SPLIT ? 64 : TW * TH / 2, SPLIT ? 8 : CKPT ? 4
             }
             const V alpha = L::make(am);
             const V w = mul2(alpha, T);
-            C0 = fma2(L::of(E.r), w, C0);  // blend_accum; the colours were clamped at staging
-            C1 = fma2(L::of(E.g), w, C1);
-            C2 = fma2(L::of(E.b), w, C2);
+            auto add = [&](V& sum, float2 c) {  // blend_accum; the colours were clamped at staging
+              const V more = fma2(L::of(c), w, sum);
+              sum = FINITE ? more : L::pick(take[u], more, sum);
+            };
+            add(C0, E.r);
+            add(C1, E.g);
+            add(C2, E.b);
             if constexpr (CKPT) {
-              S0 = fma2(L::of(E.r), w, S0);
-              S1 = fma2(L::of(E.g), w, S1);
-              S2 = fma2(L::of(E.b), w, S2);
+              add(S0, E.r);
+              add(S1, E.g);
+              add(S2, E.b);
             }
             T = mul2(T, add2(L::all(1.f), neg2(alpha)));
             if (any) E.hit[SPLIT ? 0 : warp] = 1;
@@ -705,15 +723,14 @@ __global__ void __launch_bounds__(SPLIT ? 64 : TW * TH / 2, SPLIT ? 8 : CKPT ? 4
     uint32_t top = s_work;
     if (SPLIT) {
       // The last of the tile's four CTAs knows the tile's.
-      __shared__ uint32_t s_top;
       if (threadIdx.x == 0) {
         uint32_t* sync = a.b.tile_sync + 2 * (size_t)item;
         atomicMax(sync, top);
         __threadfence();
-        s_top = atomicAdd(sync + 1, 1u) == 3u ? atomicMax(sync, 0u) : 0xffffffffu;
+        S.top = atomicAdd(sync + 1, 1u) == 3u ? atomicMax(sync, 0u) : 0xffffffffu;
       }
       __syncthreads();
-      top = s_top;
+      top = S.top;
     }
     if (!SPLIT || top != 0xffffffffu) {
       const uint32_t cost = top > s0 ? top - s0 : 0u;
@@ -737,6 +754,16 @@ __global__ void __launch_bounds__(SPLIT ? 64 : TW * TH / 2, SPLIT ? 8 : CKPT ? 4
     __syncthreads();
     if (threadIdx.x == 0) s_work = 0u;
   }
+}
+
+template <int TW, int TH, int BATCH, bool CKPT, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 64 : TW * TH / 2, SPLIT ? 8 : CKPT ? 4 : kFwdThreadsPerSm / (TW * TH / 2))
+    raster_fwd_kernel(RasterArgs a) {
+  __shared__ FwdSmem<BATCH, SPLIT ? 2 : TW * TH / 64> S;
+  if (!SPLIT && *a.b.inf_colour == 0u)
+    blend_items<TW, TH, BATCH, CKPT, SPLIT, true>(a, S);
+  else
+    blend_items<TW, TH, BATCH, CKPT, SPLIT, false>(a, S);
 }
 
 // Reduce-scatter of 12 per-lane values over the warp in 13 shuffles. Lane
