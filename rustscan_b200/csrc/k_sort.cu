@@ -338,11 +338,11 @@ constexpr int kClusterWarps = kClusterThreads / 32;
 constexpr int kClusterDigits = 512;  // of at most 9 bits
 // Up to 13 pairs per thread of 16 CTAs, and for more than 4 views (the GPU
 // holds about so many of these clusters at a time) few enough pairs that the
-// later waves stay cheap. Depth order and offsets by the radix passes (as they
-// were when this line was drawn) and by the cluster, in us: one view of 14k
-// visible Gaussians 85 and 34, of 55k 93 and 42, of 149k 102 and 75, of 179k
-// 97 and 98; 8 views of 55k 106 and 71, of 97k 116 and 97, of 149k 143 and
-// 153; 16 views of 55k 118 and 119.
+// later waves stay cheap. Depth order and offsets by the radix passes and by the
+// cluster, in us, all Gaussians visible: one view of 20k 73 and 28, of 60k 81 and
+// 40, of 120k 91 and 58, of 160k 93 and 73, of 213k 103 and 87; 4 views of 60k 95
+// and 40, of 213k 115 and 87; 8 views of 60k 116 and 69, of 100k 120 and 97, of 140k
+// 125 and 126 (of 200k, past the line, 156 and 157); 16 views of 60k 139 and 101.
 constexpr uint32_t kClusterMaxKeys = 16u * kClusterThreads * 13u;
 constexpr uint64_t kClusterMaxWaveKeys = 300000;
 
