@@ -405,7 +405,7 @@ void project_backward_all(const FwdState<F>& st, const BwdOut<F>& bo, bool exact
     V3<F> vcon{sg.v_conic[0], sg.v_conic[1], sg.v_conic[2]};
     V3<F> vcol{sg.v_rgb[0], sg.v_rgb[1], sg.v_rgb[2]};
     const ParamGrad<F> pg = project_backward(st.cam, mean, q, ls, sp.raw_opac[g], st.cov_blur, vxy, vcon, vcol,
-                                             sg.v_opac, sp.degree, coeff, exact, true, st.hp);
+                                             sg.v_opac, sp.degree, coeff, exact, st.hp);
     // helpers.wgsl:289-380: SH coefficient gradients.
     F b[25];
     sh_basis<F>(sp.degree, pg.viewdir.x, pg.viewdir.y, pg.viewdir.z, b);

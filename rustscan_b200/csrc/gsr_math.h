@@ -1017,13 +1017,11 @@ GSR_HD V3<F> sh_viewdir_vjp(const Cam<F>& cam, V3<F> mean, V3<F> vd, int degree,
 
 // exact == false reproduces the reference approximations (see above);
 // hp selects the FP64 compensation and inversion of the forward's
-// high-precision conic mode;
-// sh_dir == false leaves out only the view-direction term even when exact
-// (callers that add sh_viewdir_vjp themselves).
+// high-precision conic mode.
 template <class F, class Coeff>
 GSR_HD ParamGrad<F> project_backward(const Cam<F>& cam, V3<F> mean, V4<F> quat_unorm, V3<F> log_scale, F raw_opac,
                                      F cov_blur, V2<F> v_xy, V3<F> v_conic, V3<F> v_color, F v_opac, int degree,
-                                     const Coeff& coeff, bool exact, bool sh_dir = true, bool hp = false) {
+                                     const Coeff& coeff, bool exact, bool hp = false) {
   ParamGrad<F> g;
   const V3<F> vd = view_dir(cam, mean);
   g.viewdir = vd;
@@ -1080,7 +1078,7 @@ GSR_HD ParamGrad<F> project_backward(const Cam<F>& cam, V3<F> mean, V4<F> quat_u
   g.v_log_scale.z = v_scale.z * scale.z;
   g.v_quat = normalize_vjp_apply(quat_unorm, quat_to_mat3_vjp(quat, rot_scale(v_m, scale)));
   g.v_mean = mulv(transpose(cam.rot), v_mc);
-  if (exact && sh_dir && degree > 0) {
+  if (exact && degree > 0) {
     const V3<F> vm = sh_viewdir_vjp(cam, mean, vd, degree, v_color, coeff);
     g.v_mean.x = g.v_mean.x + vm.x;
     g.v_mean.y = g.v_mean.y + vm.y;

@@ -2,9 +2,9 @@
 // reverse-walk adjoint.
 //
 // One CTA per (view, tile) work item across all views of the launch. Each
-// warp owns an 8 x 4*PPL pixel block of the tile; each lane owns PPL pixels
-// of one column (rows y, y+4, ...), so the per-Gaussian terms a*dx*dx and
-// 2b*dx are formed once for all of them. The tile's depth-sorted list is staged in
+// warp owns an 8x8 pixel block of the tile (or strips and whole tiles, see the
+// kernels); each lane owns pixels of one column (rows y, y+4, ...), so the
+// per-Gaussian terms a*dx*dx and 2b*dx are formed once for all of them. The tile's depth-sorted list is staged in
 // shared memory batch by batch; while staging, the smallest sigma over each
 // warp block's rectangle gives a bit per block that the Gaussian's
 // {sigma <= log(255*opacity) + 1e-3} ellipse can reach (reached_blocks).
@@ -51,14 +51,12 @@ namespace gsr {
 
 namespace {
 
-// Pixels per lane. The forward gains nothing from more than 2. The
+// Pixels per lane: the forward gains nothing from more than 2. The
 // backward of 16x16 tiles runs one warp per tile, or per segment of a tile's
 // list, with 8 pixels per lane (raster_bwd_tile_kernel), so that each
 // Gaussian's warp reduction serves the whole tile; the other tile shapes run
 // raster_bwd_kernel with 2.
-constexpr int kFwdPPL = 2;
-static_assert(4 * kFwdPPL == 8, "forward warp blocks, and so the exported hit bits, are 8x8 pixels");
-constexpr int kBwdPPL = 2;
+
 // The one-warp backward's batch (entries staged per round, double-buffered)
 // and its resident CTAs per SM: 64 entries take 13 KB of shared memory, so
 // that 16 CTAs fit an SM, the register bound of 16 (at most 128 a thread).
@@ -204,14 +202,13 @@ __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(ViewSet vs, 
     b.sched_order[atomicAdd(&s_start[cost_bucket(cost_of(i))], 1u)] = i;
 }
 
-// Warp w of a TW-wide tile owns the 8 x (4*PPL) block at (x0, y0); lane l
-// owns column x0 + (l & 7) and rows y0 + (l >> 3) + 4q, q = 0..PPL-1.
-template <int TW, int PPL> struct WarpBlock {
+// Block w of a TW-wide tile is the 8x8 pixels at (x0, y0); a warp's lane l owns
+// its column x0 + (l & 7) and rows y0 + (l >> 3) + {0, 4}.
+template <int TW> struct WarpBlock {
   static_assert(TW % 8 == 0, "tile width is a multiple of the 8-pixel warp block");
   static constexpr int kWarpsX = TW / 8;
-  static constexpr int kRows = 4 * PPL;
   __device__ static int x0(int w) { return (w % kWarpsX) * 8; }
-  __device__ static int y0(int w) { return (w / kWarpsX) * kRows; }
+  __device__ static int y0(int w) { return (w / kWarpsX) * 8; }
 };
 
 // The warp blocks (8 columns, ROWS rows) of a tile at (tx0, ty0) that a
@@ -470,8 +467,8 @@ __device__ __forceinline__ void blend_items(const RasterArgs& a, FwdSmem<BATCH, 
     const ViewDesc& vd = a.vs.views[v];
     const uint32_t t = item - vd.tile_base;
     const uint32_t tx = t % vd.tiles_x, ty = t / vd.tiles_x;
-    const uint32_t px = tx * TW + WarpBlock<TW, 2>::x0(block) + (lane & 7);
-    const uint32_t py = ty * TH + WarpBlock<TW, 2>::y0(block) + (lane >> 3) + 4 * half;
+    const uint32_t px = tx * TW + WarpBlock<TW>::x0(block) + (lane & 7);
+    const uint32_t py = ty * TH + WarpBlock<TW>::y0(block) + (lane >> 3) + 4 * half;
     const float pcx = (float)px + 0.5f;
     float rows[PX], first[PX];
     bool inside[PX];
@@ -490,8 +487,8 @@ __device__ __forceinline__ void blend_items(const RasterArgs& a, FwdSmem<BATCH, 
     uint8_t* vis = slice(a.b.visible_c, a.b.Vcap, v);
     uint8_t* hitw = slice(a.b.hitw, a.b.Icap, v);
     // Corner of the CTA's pixel area.
-    const float tx0 = (float)(tx * TW + (SPLIT ? WarpBlock<TW, 2>::x0(block) : 0));
-    const float ty0 = (float)(ty * TH + (SPLIT ? WarpBlock<TW, 2>::y0(block) : 0));
+    const float tx0 = (float)(tx * TW + (SPLIT ? WarpBlock<TW>::x0(block) : 0));
+    const float ty0 = (float)(ty * TH + (SPLIT ? WarpBlock<TW>::y0(block) : 0));
     V T = L::make(first), C0 = L::all(0.f), C1 = C0, C2 = C0;
     uint32_t last[PX] = {}, nc[PX] = {};
     auto saturated = [&] {
@@ -974,31 +971,6 @@ __device__ __forceinline__ void bwd_pair_rest(BwdPair& p, const PairPre& q, floa
   }
 }
 
-// Maps the forward's per-entry warp-block bits (blocks of kFwdPPL pixels
-// per lane) onto the warp blocks of a backward with PB pixels per lane: a
-// backward block is the union of the forward blocks of its column span and
-// rows.
-// The forward warp block (8x8 pixels) that holds pixel pair k of backward
-// warp w with PB pixels per lane (its rows 8k .. 8k + 7).
-template <int TW, int PB>
-__device__ __forceinline__ int fwd_block_of(int w, int k) {
-  constexpr int KX = TW / 8;
-  return (w % KX) + ((w / KX) * (PB / 2) + k) * KX;
-}
-
-template <int TW, int TH, int PB>
-__device__ __forceinline__ uint32_t hit_bits_for(uint32_t f) {
-  constexpr int PF = kFwdPPL;
-  static_assert(PB % PF == 0, "backward warp blocks are unions of forward ones");
-  constexpr int NWF = TW * TH / PF / 32;
-  constexpr int KX = TW / 8;
-  if (PB == PF) return f;
-  uint32_t m = 0;
-#pragma unroll
-  for (int fw = 0; fw < NWF; ++fw) m |= ((f >> fw) & 1u) << ((fw % KX) + ((fw / KX) * PF / PB) * KX);
-  return m;
-}
-
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
@@ -1010,18 +982,17 @@ __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_g
 // index down in batches. Batches are double-buffered: while batch k is
 // evaluated, the raw records of batch k + 1 are in flight (asynchronous
 // copies into the other buffer) and the list entries of batch k + 2 (hit
-// bits and compact indices) are loaded into registers.
-template <int TW, int TH, int PPL, int BATCH, bool REF>
-__global__ void __launch_bounds__(TW* TH / PPL) raster_bwd_kernel(RasterArgs a) {
-  static_assert(PPL % 2 == 0, "pixels per lane come in pairs");
-  static_assert(TH % (4 * PPL) == 0 && (TW * TH / PPL) % 32 == 0, "warp blocks tile the tile");
-  constexpr int NT = TW * TH / PPL;
+// bits and compact indices) are loaded into registers. A warp owns one of the
+// forward's 8x8 blocks, a lane a pixel pair of it.
+template <int TW, int TH, int BATCH, bool REF>
+__global__ void __launch_bounds__(TW* TH / 2) raster_bwd_kernel(RasterArgs a) {
+  static_assert(TW % 8 == 0 && TH % 8 == 0, "warp blocks tile the tile");
+  constexpr int NT = TW * TH / 2;
   constexpr int NW = NT / 32;
-  constexpr int NP = PPL / 2;
   constexpr int kSI = (BATCH + NT - 1) / NT;  // entries a thread stages per batch
   __shared__ float4 s_rec[2][BATCH][3];        // raw records
   __shared__ uint32_t s_cidx[2][BATCH];
-  __shared__ uint8_t s_mask[2][BATCH];         // warp blocks that take the entry
+  __shared__ uint8_t s_mask[2][BATCH];         // blocks, and so warps, that take the entry
   __shared__ uint16_t s_list[NW][BATCH];
   __shared__ float4 s_part[NW][BATCH][3];      // written by the warps whose bit is set
   __shared__ uint32_t s_max;
@@ -1036,8 +1007,8 @@ __global__ void __launch_bounds__(TW* TH / PPL) raster_bwd_kernel(RasterArgs a) 
     const uint32_t t = item - vd.tile_base;
     const uint32_t tx = t % vd.tiles_x, ty = t / vd.tiles_x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t px = tx * TW + WarpBlock<TW, PPL>::x0(warp) + (lane & 7);
-    const uint32_t pyb = ty * TH + WarpBlock<TW, PPL>::y0(warp) + (lane >> 3);
+    const uint32_t px = tx * TW + WarpBlock<TW>::x0(warp) + (lane & 7);
+    const uint32_t pyb = ty * TH + WarpBlock<TW>::y0(warp) + (lane >> 3);
     const float pcx = (float)px + 0.5f;
     const uint32_t* ranges = slice(a.b.ranges, 2 * a.b.Tcap, v);
     const uint32_t s0 = ranges[2 * t];
@@ -1047,13 +1018,9 @@ __global__ void __launch_bounds__(TW* TH / PPL) raster_bwd_kernel(RasterArgs a) 
     const uint8_t* hitw = slice(a.b.hitw, a.b.Icap, v);
     float4* sgrad = slice(a.b.sgrad, a.b.Vcap * 3, v);
     float* part = a.b.sgrad_part + (size_t)a.b.Icap * 12 * v;
-    BwdPair pp[NP];
-    uint32_t mylast = 0;
-  #pragma unroll
-    for (int k = 0; k < NP; ++k) {
-      load_bwd_pair(a, vd, v, px, pyb + 8 * k, pp[k]);
-      mylast = max(mylast, max(pp[k].last0, pp[k].last1));
-    }
+    BwdPair pp;
+    load_bwd_pair(a, vd, v, px, pyb, pp);
+    const uint32_t mylast = max(pp.last0, pp.last1);
     if (threadIdx.x == 0) s_max = 0;
     __syncthreads();
     const uint32_t wmax = __reduce_max_sync(0xffffffffu, mylast);
@@ -1062,10 +1029,6 @@ __global__ void __launch_bounds__(TW* TH / PPL) raster_bwd_kernel(RasterArgs a) 
     const uint32_t smax = s_max;
     const int slot = reduce12_slot(lane);                          // the gradient value this lane ends with
     const bool writer = (lane & 1) == 0 && !((lane & 2) && (lane & 4));  // one lane per value
-    uint32_t wsel = 0;  // the forward blocks inside this warp's block
-  #pragma unroll
-    for (int k = 0; k < NP; ++k) wsel |= 1u << fwd_block_of<TW, PPL>(warp, k);
-    const uint32_t b0 = fwd_block_of<TW, PPL>(warp, 0);
     auto batch_lo = [&](uint32_t e) { return (e - s0 > (uint32_t)BATCH) ? e - BATCH : s0; };
     // List entries [lo, hi) of a batch into registers.
     uint32_t pc[kSI], ph[kSI];
@@ -1116,7 +1079,7 @@ __global__ void __launch_bounds__(TW* TH / PPL) raster_bwd_kernel(RasterArgs a) 
       cp_async_wait1();  // this thread's copies of the current batch have landed
       __syncthreads();
       if (bs < wmax) {
-        const int cnt = build_list(s_mask[buf], nb, wsel, lane, s_list[warp]);
+        const int cnt = build_list(s_mask[buf], nb, 1u << warp, lane, s_list[warp]);
         for (int e = cnt - 1; e >= 0; --e) {
           const uint32_t j = s_list[warp][e];
           const uint32_t s = bs + j;
@@ -1129,47 +1092,13 @@ __global__ void __launch_bounds__(TW* TH / PPL) raster_bwd_kernel(RasterArgs a) 
           const float t2 = emul(A.w, dx);
           const float cb = r0.w;  // the conic's b
           const float adx = A.z * dx, bdx = cb * dx;
-          BwdMom mom;  // set by the first pair evaluated
+          BwdMom mom;
           BwdAcc acc;
           const float cp0 = fmaxf(Cc.x, 0.f), cp1 = fmaxf(Cc.y, 0.f), cp2 = fmaxf(Cc.z, 0.f);
-          // The pairs of this warp whose 8x8 block had a pixel take the
-          // Gaussian in the forward (the others contribute nothing here).
-          const uint32_t mraw = s_mask[buf][j];
-          // Pair k takes part when its forward block took the Gaussian (a
-          // warp-uniform test); the first pair evaluated sets the sums.
-          auto rest = [&](int k, auto first) {
-            const float2 npcy = make_float2(-((float)(pyb + 8 * k) + 0.5f), -((float)(pyb + 8 * k + 4) + 0.5f));
-            const PairPre pre = bwd_pair_pre(pp[k], npcy, s, t1, t2, A, B);
-            const float2 cpv =
-                fma2(f2(cp2), pp[k].vb, fma2(f2(cp1), pp[k].vg, mul2(f2(cp0), pp[k].vr)));
-            constexpr bool kF = decltype(first)::value;
-            bwd_pair_rest<REF, kF, kF>(pp[k], pre, adx, bdx, cb, B, cpv, pp[k].vr, pp[k].vg, pp[k].vb, mom, acc);
-          };
-          constexpr std::integral_constant<bool, true> kFirst{};
-          constexpr std::integral_constant<bool, false> kNext{};
-          if constexpr (NP == 1) {
-            rest(0, kFirst);  // listed entries take part in the warp's one pair
-          } else if constexpr (NP == 2) {
-            // Pair k of this warp lies in forward block b0 + k * KX; the
-            // needed pairs run as one straight-line block, so that their
-            // independent chains interleave.
-            constexpr uint32_t KX = TW / 8, both = 1u | (1u << KX);
-            const uint32_t need = (mraw >> b0) & both;  // listed entries have at least one
-            if (need == both) {
-              rest(0, kFirst);
-              rest(1, kNext);
-            } else if (need == 1u) {
-              rest(0, kFirst);
-            } else {
-              rest(1, kFirst);
-            }
-          } else {
-            mom.m0 = mom.m1 = mom.m2 = acc.cr = acc.cg = acc.cb = acc.ax = acc.ay = f2(0.f);
-            acc.n = 0u;
-  #pragma unroll
-            for (int k = 0; k < NP; ++k)
-              if ((mraw >> fwd_block_of<TW, PPL>(warp, k)) & 1u) rest(k, kNext);
-          }
+          const float2 npcy = make_float2(-((float)pyb + 0.5f), -((float)(pyb + 4) + 0.5f));
+          const PairPre pre = bwd_pair_pre(pp, npcy, s, t1, t2, A, B);
+          const float2 cpv = fma2(f2(cp2), pp.vb, fma2(f2(cp1), pp.vg, mul2(f2(cp0), pp.vr)));
+          bwd_pair_rest<REF, true, true>(pp, pre, adx, bdx, cb, B, cpv, pp.vr, pp.vg, pp.vb, mom, acc);
           const float M0 = mom.m0.x + mom.m0.y, M1 = mom.m1.x + mom.m1.y, M2 = mom.m2.x + mom.m2.y;
           float x[12];
           x[0] = dx * M0;  // S1..S5 (the conic combination follows the CTA sum)
@@ -1192,7 +1121,7 @@ __global__ void __launch_bounds__(TW* TH / PPL) raster_bwd_kernel(RasterArgs a) 
       __syncthreads();
       for (uint32_t q = threadIdx.x; q < nb * 3; q += NT) {
         const uint32_t j = q / 3, k = q % 3;
-        const uint32_t m = hit_bits_for<TW, TH, PPL>(s_mask[buf][j]);  // warps that wrote a slot
+        const uint32_t m = s_mask[buf][j];  // warps that wrote a slot
         float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
         bool any = false;
   #pragma unroll
@@ -1569,25 +1498,25 @@ cudaError_t launch_fwd_16(const RasterArgs& a, uint32_t batch, int num_sms, cuda
     default: return launch_fwd_batch<16, 16, 256, true, false>(a, num_sms, st);
   }
 }
-template <int TW, int TH, int PPL, bool REF>
+template <int TW, int TH, bool REF>
 cudaError_t launch_bwd_mode(const RasterArgs& a, uint32_t batch, int num_sms, cudaStream_t st) {
-  constexpr int NT = TW * TH / PPL;
+  constexpr int NT = TW * TH / 2;
   constexpr int kMaxBatch = NT / 32 >= 2 ? 128 : 256;
   const uint32_t items = a.vs.total_tiles;
   int b = pick_batch(batch, 64);
   if (b > kMaxBatch) b = kMaxBatch;
   switch (b) {
-    case 64: return launch_items<raster_bwd_kernel<TW, TH, PPL, 64, REF>>(NT, a, items, num_sms, st);
-    case 128: return launch_items<raster_bwd_kernel<TW, TH, PPL, 128, REF>>(NT, a, items, num_sms, st);
+    case 64: return launch_items<raster_bwd_kernel<TW, TH, 64, REF>>(NT, a, items, num_sms, st);
+    case 128: return launch_items<raster_bwd_kernel<TW, TH, 128, REF>>(NT, a, items, num_sms, st);
     default:
-      return launch_items<raster_bwd_kernel<TW, TH, PPL, (kMaxBatch > 128 ? 256 : 128), REF>>(NT, a, items, num_sms,
-                                                                                               st);
+      return launch_items<raster_bwd_kernel<TW, TH, (kMaxBatch > 128 ? 256 : 128), REF>>(NT, a, items, num_sms,
+                                                                                          st);
   }
 }
-template <int TW, int TH, int PPL>
+template <int TW, int TH>
 cudaError_t launch_bwd_shape(const RasterArgs& a, uint32_t batch, int num_sms, cudaStream_t st) {
-  return a.ref_mode ? launch_bwd_mode<TW, TH, PPL, true>(a, batch, num_sms, st)
-                    : launch_bwd_mode<TW, TH, PPL, false>(a, batch, num_sms, st);
+  return a.ref_mode ? launch_bwd_mode<TW, TH, true>(a, batch, num_sms, st)
+                    : launch_bwd_mode<TW, TH, false>(a, batch, num_sms, st);
 }
 // 16x16 tiles: one warp per (tile, segment). It stages 64 entries per batch
 // whatever the forward's batch: 13 KB of shared memory and at most 128
@@ -1634,10 +1563,10 @@ void raster_warm_up(uint32_t tile_w, uint32_t tile_h, uint32_t batch, int num_sm
       (void)launch_bwd_16(a, num_sms, nullptr);
     } else if (tile_w == 8 && tile_h == 8) {
       (void)launch_fwd_shape<8, 8>(a, batch, num_sms, nullptr);
-      (void)launch_bwd_shape<8, 8, kBwdPPL>(a, batch, num_sms, nullptr);
+      (void)launch_bwd_shape<8, 8>(a, batch, num_sms, nullptr);
     } else if (tile_w == 32 && tile_h == 8) {
       (void)launch_fwd_shape<32, 8>(a, batch, num_sms, nullptr);
-      (void)launch_bwd_shape<32, 8, kBwdPPL>(a, batch, num_sms, nullptr);
+      (void)launch_bwd_shape<32, 8>(a, batch, num_sms, nullptr);
     }
   }
 }
@@ -1703,8 +1632,8 @@ cudaError_t launch_raster_bwd(const ViewSet& vs, FwdBufs& b, const float* bg, co
     if (e != cudaSuccess) return e;
   }
   if (vs.tile_w == 16 && vs.tile_h == 16) return launch_bwd_16(a, s.num_sms, st);
-  if (vs.tile_w == 8 && vs.tile_h == 8) return launch_bwd_shape<8, 8, kBwdPPL>(a, vs.batch, s.num_sms, st);
-  if (vs.tile_w == 32 && vs.tile_h == 8) return launch_bwd_shape<32, 8, kBwdPPL>(a, vs.batch, s.num_sms, st);
+  if (vs.tile_w == 8 && vs.tile_h == 8) return launch_bwd_shape<8, 8>(a, vs.batch, s.num_sms, st);
+  if (vs.tile_w == 32 && vs.tile_h == 8) return launch_bwd_shape<32, 8>(a, vs.batch, s.num_sms, st);
   return cudaErrorInvalidValue;
 }
 
