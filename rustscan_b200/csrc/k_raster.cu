@@ -137,10 +137,12 @@ __device__ __forceinline__ uint32_t next_item(const RasterArgs& a, uint32_t roun
     return at < a.vs.total_tiles ? a.b.sched_order[at] * PARTS + slot % PARTS : kNoItem;
   });
 }
-// FIRST (launches whose items fit the resident CTAs a few times over): a CTA's
-// first place is its own index, without a ticket, and warp 0's lanes look
-// through the lists at once, because there an item's start is a good part of
-// its time.
+// FIRST (launches whose items fit the resident CTAs a few times over, and tiles
+// of several warps or few pixels): a CTA's first place is its own index, without a
+// ticket, and warp 0's lanes look through the lists at once, because there an
+// item's start is a good part of its time. Backward of 8x8 tiles, one view of
+// 639x479 over 200k Gaussians, 164 us without and 146 with it, of 32x8 tiles 242
+// and 195, 4 views of 1280x720 over 300k in 32x8 tiles 957 and 930.
 template <bool FIRST>
 __device__ __forceinline__ uint32_t next_item(const RasterArgs& a, uint32_t round, uint32_t* s_item,
                                               const CostListView* lists) {
@@ -1000,7 +1002,7 @@ __global__ void __launch_bounds__(TW* TH / 2) raster_bwd_kernel(RasterArgs a) {
   __shared__ CostListView s_lists;
   load_cost_lists(a, &s_lists);
   for (uint32_t round = 0;; ++round) {
-    const uint32_t item = next_item<false>(a, round, &s_item, &s_lists);
+    const uint32_t item = next_item<true>(a, round, &s_item, &s_lists);
     if (item == kNoItem) break;
     const uint32_t v = find_view(a.vs, item);
     const ViewDesc& vd = a.vs.views[v];
