@@ -202,7 +202,7 @@ gsr_status allocate(gsr_ctx* c) {
       cudaMemset(b.vcount, 0, sizeof(uint32_t) * 4 * nv) != cudaSuccess ||
       cudaMemset(b.sched_lcount, 0, sizeof(uint32_t) * kSchedWords) != cudaSuccess)
     return cuda_fail(c, cudaGetLastError(), "cudaMemset");
-  raster_warm_up(cfg.tile_w, cfg.tile_h, cfg.batch, c->num_sms);
+  raster_warm_up(cfg.tile_w, cfg.tile_h, cfg.batch, cfg.deterministic, c->num_sms);
   return GSR_OK;
 }
 
