@@ -92,7 +92,7 @@ __device__ __forceinline__ void load_view(const ViewDesc& d, BwdView& o) {
 // adds into the gradients of the mean and, as the symmetric matrix (xx, xy, xz,
 // yy, yz, zz), of the 3D covariance, returns the opacity logit's. Written out
 // for the symmetric matrices and the Jacobian's zeros, which the general
-// functions multiply through.
+// functions multiply through; divisions and roots are correctly rounded, as there.
 struct ViewAdjoint {
   V3<float> v_mean;
   float v_cov[6];
@@ -275,9 +275,9 @@ __device__ __forceinline__ void stage_sh_rows(const __nv_bfloat16* src, uint32_t
 }
 
 // One thread per Gaussian. What bounds it: the latency of its loads at 16 warps
-// per SM (128 registers, 48 of them the SH sums; fewer registers spill, a third
-// record stage or a fourth of the blocks less costs more than it hides), at 0.4
-// of the DRAM rate and of the issue slots each. It replaces a pass per (view,
+// per SM (128 registers, 48 of them the SH sums; degree 3 spills 124 bytes, fewer
+// registers spill more, and a third record stage or a fourth of the blocks less
+// costs more than it hides), at 0.4 of the DRAM rate and of the issue slots each. It replaces a pass per (view,
 // Gaussian) that wrote 96-byte adjoint records, a pass that summed them and, in
 // a training step, the Adam passes that read the gradient back: 8 views of 1M
 // Gaussians 0.817 -> 0.626 ms, 16 uneven views of 2M (BF16 SH) 2.77 -> 1.82, one

@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(ScanArgs a) {
 // stably (as sort_pass_kernel does), the CTAs send their digit counts to one
 // another, and every pair is stored straight to its place in the CTA that
 // owns it. Two cluster barriers per pass take the place of a launch and a
-// look-back. What bounds it is latency: about 2000 cycles per barrier, and per
+// look-back (another, that every CTA has started, hides behind the key loads). What bounds it is latency: about 2000 cycles per barrier, and per
 // 1024 pairs of a CTA 1300 to send them (single 8-byte stores) besides the
 // ranking.
 // ---------------------------------------------------------------------------
